@@ -47,13 +47,9 @@ struct BdArgs {
 
 __device__ __forceinline__ float3 mind(const BdArgs &a, int i, int j) {
     const SysDev &sd = a.sys[a.atom_sys[i]];  // a term never spans two systems
-    double d[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        d[k] = a.x[3 * j + k] - a.x[3 * i + k];
-        d[k] -= sd.Ld[k] * rint(d[k] * sd.invLd[k]);
-    }
-    return make_float3((float)d[0], (float)d[1], (float)d[2]);
+    return make_float3(min_image(sd, a.x[3 * j], a.x[3 * i], 0),
+                       min_image(sd, a.x[3 * j + 1], a.x[3 * i + 1], 1),
+                       min_image(sd, a.x[3 * j + 2], a.x[3 * i + 2], 2));
 }
 
 __device__ __forceinline__ void addf(const BdArgs &a, int atom, float fx, float fy, float fz) {
@@ -88,6 +84,9 @@ __device__ float torsion(const BdArgs &a, int4 id, float3 g[4], bool &ok) {
     return phi;
 }
 
+// ENERGY: only an evaluation that reports energies sums them (FP64 warp sums:
+// a third of this kernel's FP64-pipe time otherwise)
+template <bool ENERGY>
 __global__ void __launch_bounds__(256) k_bonded(BdArgs a) {
     const int b = blockIdx.x;
     int seg = 0;
@@ -172,6 +171,7 @@ __global__ void __launch_bounds__(256) k_bonded(BdArgs a) {
             addf(a, id.w, -dv * g[3].x, -dv * g[3].y, -dv * g[3].z);
         }
     }
+    if (!ENERGY) return;
     const double v[1] = {(double)e};
     const int slot[1] = {MDG_TERM_BOND + seg};
     block_energy_add<1>(a.energy, first >= 0 ? a.atom_sys[first] : -1, v, slot);
@@ -180,7 +180,6 @@ __global__ void __launch_bounds__(256) k_bonded(BdArgs a) {
 }  // namespace
 
 cudaError_t launch_bonded(mdg_system *s, unsigned mask, int energy) {
-    (void)energy;
     BdArgs a;
     a.x = s->x;
     a.inv_perm = s->inv_perm;
@@ -208,7 +207,8 @@ cudaError_t launch_bonded(mdg_system *s, unsigned mask, int energy) {
     a.f = s->f;
     a.n_pad = s->n_pad;
     a.energy = s->energy;
-    k_bonded<<<a.blk_end, tb, 0, s->stream>>>(a);
+    if (energy) k_bonded<true><<<a.blk_end, tb, 0, s->stream>>>(a);
+    else k_bonded<false><<<a.blk_end, tb, 0, s->stream>>>(a);
     s->launches += 1;
     return cudaGetLastError();
 }

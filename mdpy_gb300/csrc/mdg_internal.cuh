@@ -129,6 +129,20 @@ __device__ void block_energy_add(long long *energy, int sys, const double (&v)[N
 
 struct SysDev;
 
+// Component k of the FP64 minimum-image difference x_j - x_i, rounded to FP32.
+// The image is decided in FP32 where that is certain (|d| below 0.4999 L): one
+// FP64 subtraction and one conversion instead of five FP64-pipe operations.
+template <class Sys>
+__device__ __forceinline__ float min_image(const Sys &sd, double xj, double xi, int k) {
+    double d = xj - xi;
+    float f = (float)d;
+    if (fabsf(f * sd.invL[k]) > 0.4999f) {
+        d -= sd.Ld[k] * rint(d * sd.invLd[k]);
+        f = (float)d;
+    }
+    return f;
+}
+
 // Per-step packing of one 32-slot cluster into the float copy the force
 // kernels read (see pack_cluster below).
 struct PackArgs {
@@ -152,6 +166,7 @@ struct SysDev {
     float L[3], invL[3];    // box edges (A) and inverses
     double Ld[3];           // FP64 box for the FP64 minimum image
     double invLd[3];        // and its inverse (GB300's FP64 divide is slow)
+    double ncl[3];          // sort columns and height bins per A
     int atom_off, n_atoms;  // atom range
     int cl_off, cl_cap;     // cluster range (capacity: ceil(n/32) + columns)
     int col_off, n_cols;    // sort columns
@@ -229,11 +244,20 @@ __device__ __forceinline__ void pack_cluster(const PackArgs &a, int warp, int k,
     const int lane = threadIdx.x & 31;
     float4 p;
     if (valid) {
-        const double *Ld = a.sys[a.cl_sys[warp]].Ld;
+        // (decided in FP32 where that is certain: FP64 operations run at two
+        // lanes per clock and SM)
+        const SysDev &sd = a.sys[a.cl_sys[warp]];
+        float cf[3];
 #pragma unroll
-        for (int d = 0; d < 3; ++d)
-            if (c[d] < -0.25 * Ld[d] || c[d] >= 1.25 * Ld[d]) c[d] -= Ld[d] * floor(c[d] / Ld[d]);
-        p = make_float4((float)c[0], (float)c[1], (float)c[2], a.q_sorted[k]);
+        for (int d = 0; d < 3; ++d) {
+            cf[d] = (float)c[d];
+            if (!(cf[d] > -0.249f * sd.L[d] && cf[d] < 1.249f * sd.L[d])) {
+                const double Ld = sd.Ld[d];
+                if (c[d] < -0.25 * Ld || c[d] >= 1.25 * Ld) c[d] -= Ld * floor(c[d] / Ld);
+                cf[d] = (float)c[d];
+            }
+        }
+        p = make_float4(cf[0], cf[1], cf[2], a.q_sorted[k]);
     } else {
         p = make_float4(kFarAway, kFarAway, kFarAway, 0.0f);
     }

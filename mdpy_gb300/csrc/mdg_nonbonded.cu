@@ -179,7 +179,9 @@ struct SpArgs {
 // Excluded 1-2/1-3 pairs: -k q q erf(beta r)/r removes their share of the
 // reciprocal sum (term COUL_RECIP).  1-4 pairs: LJ with the 1-4 parameters
 // (charmm_nonbonded_constraint.py:92-97) and the real-space Coulomb term.
-template <bool SWITCH, bool DUMP>
+// ENERGY: only an evaluation that reports energies sums them (three FP64 warp
+// sums a thread otherwise).
+template <bool SWITCH, bool DUMP, bool ENERGY>
 __global__ void k_special(SpArgs a) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     float e_lj = 0.f, e_cr = 0.f, e_rec = 0.f;
@@ -192,11 +194,7 @@ __global__ void k_special(SpArgs a) {
         const SysDev &sd = a.sys[sid];
         float d[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            double dd = a.x[3 * j + k] - a.x[3 * i + k];
-            dd -= sd.Ld[k] * rint(dd * sd.invLd[k]);
-            d[k] = (float)dd;
-        }
+        for (int k = 0; k < 3; ++k) d[k] = min_image(sd, a.x[3 * j + k], a.x[3 * i + k], k);
         const float r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
         const float r = sqrtf(r2);
         const float qq = a.charge[i] * a.charge[j];
@@ -254,7 +252,7 @@ __global__ void k_special(SpArgs a) {
             fix_red(&ff[2 * a.n_pad + ki], to_fix(-fr * d[2]));
         }
     }
-    if (DUMP) return;
+    if (DUMP || !ENERGY) return;
     // FP64 block sums: the exclusion term is a sum of O(10^5) terms of either
     // sign whose total largely cancels the self energy
     const double v[3] = {(double)e_lj, (double)e_cr, (double)e_rec};
@@ -358,7 +356,6 @@ cudaError_t launch_nonbonded(mdg_system *s, unsigned mask, int energy, int dump)
 }
 
 cudaError_t launch_special(mdg_system *s, unsigned mask, int energy, int dump) {
-    (void)energy;
     SpArgs a;
     a.x = s->x;
     a.inv_perm = s->inv_perm;
@@ -397,11 +394,13 @@ cudaError_t launch_special(mdg_system *s, unsigned mask, int energy, int dump) {
     const bool sw = s->rswitch > 0 && s->rswitch < s->cutoff;
     const int tb = 256, nb = (total + tb - 1) / tb;
     if (dump)
-        sw ? k_special<true, true><<<nb, tb, 0, s->stream>>>(a)
-           : k_special<false, true><<<nb, tb, 0, s->stream>>>(a);
+        k_special<false, true, false><<<nb, tb, 0, s->stream>>>(a);
+    else if (energy)
+        sw ? k_special<true, false, true><<<nb, tb, 0, s->stream>>>(a)
+           : k_special<false, false, true><<<nb, tb, 0, s->stream>>>(a);
     else
-        sw ? k_special<true, false><<<nb, tb, 0, s->stream>>>(a)
-           : k_special<false, false><<<nb, tb, 0, s->stream>>>(a);
+        sw ? k_special<true, false, false><<<nb, tb, 0, s->stream>>>(a)
+           : k_special<false, false, false><<<nb, tb, 0, s->stream>>>(a);
     s->launches += 1;
     return cudaGetLastError();
 }

@@ -42,17 +42,22 @@ __global__ void k_bin(double *__restrict__ x, int n, const SysDev *__restrict__ 
     bool ok = true;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const double L = d.Ld[k];
         double p = x[3 * i + k];
-        // particle loss as mdpy's wrap_positions defines it (mdpy/utils/pbc.py:
-        // 30-34): a non-finite coordinate, or one two or more box lengths
-        // from the central image (|round(x / L)| >= 2)
-        ok = ok && isfinite(p) && fabs(rint(p * d.invLd[k])) < 2.0;
-        p -= L * floor(p / L);
-        if (p >= L) p -= L;
-        if (!(p >= 0.0)) p = 0.0;
-        x[3 * i + k] = p;
-        int b = (int)(p * (nc[k] / L));
+        // a coordinate that FP32 shows to lie inside [0, L) needs no FP64
+        // division and no wrap
+        const float pf = (float)p * d.invL[k];
+        if (!(pf > 1e-4f && pf < 0.9999f)) {
+            const double L = d.Ld[k];
+            // particle loss as mdpy's wrap_positions defines it (mdpy/utils/pbc.py:
+            // 30-34): a non-finite coordinate, or one two or more box lengths
+            // from the central image (|round(x / L)| >= 2)
+            ok = ok && isfinite(p) && fabs(rint(p * d.invLd[k])) < 2.0;
+            p -= L * floor(p / L);
+            if (p >= L) p -= L;
+            if (!(p >= 0.0)) p = 0.0;
+            x[3 * i + k] = p;
+        }
+        int b = (int)(p * d.ncl[k]);
         c[k] = b < 0 ? 0 : (b >= nc[k] ? nc[k] - 1 : b);
     }
     if (!ok) raise_status(status, MDG_ERR_PARTICLE_LOSS);
@@ -304,6 +309,9 @@ int prepare_sort_grid(mdg_system *s) {
         d.ncx = std::max(1, std::min(4096, (int)std::lround(d.Ld[0] / a)));
         d.ncy = std::max(1, std::min(4096, (int)std::lround(d.Ld[1] / a)));
         d.nzb = std::max(1, std::min(8192, (int)std::lround(d.Ld[2] / (a / 8.0))));
+        d.ncl[0] = d.ncx / d.Ld[0];
+        d.ncl[1] = d.ncy / d.Ld[1];
+        d.ncl[2] = d.nzb / d.Ld[2];
         d.n_cols = d.ncx * d.ncy;
         d.col_off = col_off;
         d.key_off = key_off;
