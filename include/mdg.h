@@ -210,7 +210,10 @@ MDG_API int mdg_step_host(mdg_system *sys, const double *x_in, const double *v_i
 /* ---- launch shapes and the autotuner (no reference counterpart) ---------
  * A launch shape is MDG_SHAPE_FIELDS ints:
  *   [MDG_SHAPE_SPLIT]          work items (one warp each) per 32-atom cluster in
- *                              the pair kernel: 1, 2, 4, 8, 16 (default 4);
+ *                              the pair kernel: 1, 2, 4, 8, 16 (default: 4; with
+ *                              Ewald 2 for each system of 128,000 atoms or more).
+ *                              Few items of small systems are taken by several
+ *                              warps each, with the same sums;
  *   [MDG_SHAPE_PERSISTENT]     0 = one CTA per work item; n = n resident CTAs
  *                              per SM (1..24) pulling work items from a device
  *                              counter (default 0);

@@ -1204,7 +1204,7 @@ static int apply_shape(mdg_system *s, const int *sh) {
 }
 
 static void current_shape(const mdg_system *s, int *sh) {
-    sh[MDG_SHAPE_SPLIT] = s->nb_split;
+    sh[MDG_SHAPE_SPLIT] = nb_parts(s);
     sh[MDG_SHAPE_PERSISTENT] = s->nb_persistent;
     sh[MDG_SHAPE_PME_BLOCK] = s->pme_block;
     sh[MDG_SHAPE_SIDE_PRIORITY] = s->side_priority;

@@ -33,6 +33,18 @@ constexpr double kFixInv = 1.0 / 4294967296.0;
 constexpr float kFarAway = 1.0e18f;
 constexpr float kFixLimit = 1.0e9f;  // |contribution| above this overflows int64 sums
 constexpr int kEnergySlots = 16;
+// The pair kernel's default number of work items per cluster, by the size of
+// the cluster's own system, so that a batch member is cut up as it is alone:
+// 4 below this many atoms, 2 from it on.  Alone on the GPU (Ewald, LJ, switch,
+// us at 2 / 4 items): 24k atoms 109 / 88, 48k 153 / 138, 88k 229 / 238, 250k
+// 560 / 625, 500k 1079 / 1188: 2 is clearly ahead only well above 100k atoms.
+constexpr int kNbLargeSystem = 128000;
+// below this many atoms a system's items may be taken by several warps (the
+// pair kernel's block form), and its sums are cut up accordingly
+constexpr int kNbBlockSystem = 8000;
+__host__ __device__ constexpr int nb_default_parts(int n_atoms) {
+    return n_atoms < kNbLargeSystem ? 4 : 2;
+}
 constexpr int kSlotKinetic = 8;
 constexpr int kStatus = 0;
 
@@ -56,6 +68,12 @@ __device__ __forceinline__ float warp_sum(float v) {
 }
 
 __device__ __forceinline__ double warp_sum_d(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+__device__ __forceinline__ long long warp_sum_ll(long long v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
@@ -503,7 +521,7 @@ struct mdg_system {
 
     // launch shapes (set by hand or by mdg_autotune): work items per
     // i-cluster, persistent work-queue form, PME spread/gather block size
-    int nb_split = 4;
+    int nb_split = 0;                 // 0: nb_default_parts of each system
     int nb_persistent = 0;            // 0: one CTA per item; else resident CTAs per SM
     int nb_persistent_ctas = 0;       // SMs x nb_persistent
     int n_sms = 0;
@@ -578,6 +596,7 @@ cudaError_t launch_reorder(mdg_system *s);
 cudaError_t launch_pack(mdg_system *s);
 PackArgs make_pack_args(mdg_system *s);
 cudaError_t launch_nonbonded(mdg_system *s, unsigned mask, int energy, int dump);
+int nb_parts(const mdg_system *s);  // work items per cluster of the pair kernel
 cudaError_t launch_special(mdg_system *s, unsigned mask, int energy, int dump);
 cudaError_t launch_pme(mdg_system *s, int energy, int *cufft_status);
 cudaError_t launch_bonded(mdg_system *s, unsigned mask, int energy);

@@ -44,6 +44,11 @@ cudaError_t launch_nb_half(mdg_system *s, const NbArgs &a, int coul_tile, bool w
 cudaError_t launch_nb_quarter(mdg_system *s, const NbArgs &a, int coul_tile, bool want_lj,
                               bool sw, int energy, int dump);  // mdg_nonbonded_quarter.cu
 
+cudaError_t launch_nb_batch(mdg_system *s, const NbArgs &a, int coul_tile, bool want_lj, bool sw,
+                            int energy);  // mdg_nonbonded_batch.cu
+cudaError_t launch_nb_block(mdg_system *s, const NbArgs &a, int warps, bool want_lj, bool sw,
+                            int energy);  // mdg_nonbonded_block.cu
+
 namespace {
 
 // Bare Coulomb over all pairs with the minimum image (parity path for
@@ -305,9 +310,10 @@ NbArgs make_args(mdg_system *s) {
     a.perm = s->perm;
     a.x = s->x;
     a.rc_ref = s->cutoff;
-    a.split = s->nb_split;
+    a.by_size = s->nb_split == 0 && s->coul_mode == MDG_COUL_EWALD;
+    a.split = nb_parts(s);
     a.persistent = s->nb_persistent > 0;
-    a.n_items = s->n_clusters * s->nb_split;
+    a.n_items = s->n_clusters * a.split;
     a.queue = s->nb_queue;
     // persistent form: one queue atomic per `grab` consecutive items, so
     // that a batch of ~10^5 items does not serialise on the counter; each
@@ -321,6 +327,16 @@ NbArgs make_args(mdg_system *s) {
 
 
 }  // namespace
+
+// work items per cluster: as set, or the most that any system's size calls for
+// (LJ without Ewald: always 4)
+int nb_parts(const mdg_system *s) {
+    if (s->nb_split > 0) return s->nb_split;
+    if (s->coul_mode != MDG_COUL_EWALD) return 4;
+    int p = 1;
+    for (const SysDev &d : s->sys_h) p = std::max(p, nb_default_parts(d.n_atoms));
+    return p;
+}
 
 cudaError_t launch_nonbonded(mdg_system *s, unsigned mask, int energy, int dump) {
     const bool want_lj = (mask & MDG_MASK(MDG_TERM_LJ)) && s->lj_on;
@@ -340,9 +356,22 @@ cudaError_t launch_nonbonded(mdg_system *s, unsigned mask, int energy, int dump)
     cudaError_t err = cudaSuccess;
     const int coul_tile = (want_c && s->coul_mode == MDG_COUL_EWALD) ? MDG_COUL_EWALD : MDG_COUL_NONE;
     if (want_lj || coul_tile == MDG_COUL_EWALD) {
-        err = s->nb_half == 2   ? launch_nb_quarter(s, a, coul_tile, want_lj, sw, energy, dump)
-              : s->nb_half == 1 ? launch_nb_half(s, a, coul_tile, want_lj, sw, energy, dump)
-                                : dispatch_shape<false>(s, a, coul_tile, want_lj, sw, energy, dump);
+        // Ewald items of small systems, too few to fill the GPU, are taken by 8,
+        // 4 or 2 warps each (the sums are the same).  Pair kernel alone, us at
+        // 1 / 2 / 4 / 8 warps: 416 items (2,700 atoms) 55 / 43 / 35 / 31, 900
+        // (6k atoms) 41 / 35 / 37 / 49; 1740 (12k) 67 / 67 / 68 / 103
+        const int warps = a.n_items <= 450 ? 8 : a.n_items <= 700 ? 4 : a.n_items <= 1200 ? 2 : 1;
+        bool small = true;
+        for (const SysDev &d : s->sys_h) small = small && d.n_atoms < kNbBlockSystem;
+        if (coul_tile == MDG_COUL_EWALD && s->nb_half == 0 && !s->nb_persistent && !dump && small &&
+            warps > 1)
+            err = launch_nb_block(s, a, warps, want_lj, sw, energy);
+        else
+            err = s->nb_half == 2   ? launch_nb_quarter(s, a, coul_tile, want_lj, sw, energy, dump)
+                  : s->nb_half == 1 ? launch_nb_half(s, a, coul_tile, want_lj, sw, energy, dump)
+                  : (s->n_sys > 1 || small) && !dump
+                      ? launch_nb_batch(s, a, coul_tile, want_lj, sw, energy)
+                                    : dispatch_shape<false>(s, a, coul_tile, want_lj, sw, energy, dump);
         s->launches += 1;
         if (err != cudaSuccess) return err;
     }

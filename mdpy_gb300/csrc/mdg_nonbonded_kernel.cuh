@@ -44,7 +44,8 @@ struct NbArgs {
     const int *perm;
     const double *x;  // FP64 state, atom order (pair dump: the reference's pair test)
     float rc_ref;     // pair dump: the cutoff of that test (the search uses rc + a margin)
-    int split;        // work items (one warp each) per i-cluster
+    int split;        // work items (one warp each) per i-cluster, at most
+    int by_size;      // 1: nb_default_parts of the cluster's system, up to split
     int persistent;   // 1: warps pull items from `queue` until none is left
     int n_items;      // n_clusters * split
     int *queue;       // next item (zeroed before each persistent launch)
@@ -456,21 +457,181 @@ __device__ __forceinline__ void pair_interact(const NbArgs &a, const SysDev &sd,
     }
 }
 
-// Candidate clusters of i-cluster I for work item `part` (of a.split): every
+__device__ __forceinline__ PairI2 pair_i2(const float4 xi, const float2 pi) {
+    PairI2 r;
+    r.X = splat2(xi.x);
+    r.Y = splat2(xi.y);
+    r.Z = splat2(xi.z);
+    r.Q = splat2(xi.w);
+    r.S = splat2(pi.x);
+    r.E = splat2(pi.y);
+    return r;
+}
+__device__ __forceinline__ PkC pk_constants(const NbArgs &a) {
+    PkC pc;
+    pc.one = splat2(1.0f);
+    pc.six = splat2(6.0f);
+    pc.twelve = splat2(12.0f);
+    pc.a1 = splat2(kAsA1);
+    pc.a2 = splat2(kAsA2);
+    pc.a3 = splat2(kAsA3);
+    pc.a4 = splat2(kAsA4);
+    pc.a5 = splat2(kAsA5);
+    pc.fc = splat2(a.ewald_fc);
+    pc.g = splat2(a.sw_g);
+#if MDG_PK_EWALD_ARGS
+    pc.bp = splat2(a.beta_p);
+    pc.negc = splat2(-a.ewald_exp_c);
+#endif
+    return pc;
+}
+
+// A lane's i-force and energy sums over an item's super-chunks.
+// EWALD, systems below kNbBlockSystem: one FP32 sum per super-chunk, int64
+// fixed point across them, so the total does not depend on which warp swept
+// which super-chunk, nor on their order (the one-warp and the block form of the
+// kernel give the same bits).  Larger systems never use the block form: one
+// FP32 chain (a conversion per super-chunk costs 2 to 3 %).
+// Otherwise (LJ alone): one FP32 chain, energies in FP64.
+template <int COUL>
+struct ItemSums {
+    unsigned n_in = 0;               // energy variant: this lane's in-cutoff pairs
+    bool per_chunk = true;           // small system: the FP32 sums end with each super-chunk
+    u64 FIX = 0ull, FIY = 0ull, FIZ = 0ull;  // +fr d, FP32
+    long long fi[3] = {0, 0, 0};     // i force
+    long long e_lj = 0, e_c = 0;
+    // F: +fr d sums of the two packed halves
+    __device__ __forceinline__ void add_force(const NbArgs &a, int axis, u64 F) {
+        float p, q;
+        unpk2(F, p, q);
+        const float v = -(p + q);
+        fi[axis] += to_fix(v);
+        // each share below 1e9 and the sum below 1e9 before it: no unnoticed wrap
+        if (!(fabsf(v) < kFixLimit) || llabs(fi[axis]) >= (long long)(1.0e9 * kFixScale))
+            raise_status(a.status, MDG_ERR_OVERFLOW);
+    }
+    __device__ __forceinline__ void end_chain(const NbArgs &a) {
+        add_force(a, 0, FIX);
+        add_force(a, 1, FIY);
+        add_force(a, 2, FIZ);
+        FIX = FIY = FIZ = 0ull;
+    }
+    __device__ __forceinline__ void push_i(const NbArgs &a, int ik) const {
+        fix_red(&a.f[ik], fi[0]);
+        fix_red(&a.f[a.n_pad + ik], fi[1]);
+        fix_red(&a.f[2 * a.n_pad + ik], fi[2]);
+    }
+};
+template <>
+struct ItemSums<MDG_COUL_NONE> {
+    unsigned n_in = 0;
+    u64 FIX = 0ull, FIY = 0ull, FIZ = 0ull;  // +fr d, negated at the end
+    double e_lj = 0.0, e_c = 0.0;
+};
+
+// One packed super-chunk (64 j atoms as 32 (A, B) pairs) at byte address sa,
+// swept in 32 rotation steps: at step t lane l pairs its i atom with pair
+// l ^ t (both halves at once), the pair's j-force accumulators travel by
+// butterfly shuffles (mask t ^ (t + 1), 31 at the end), and lane l ends with
+// pair l's two j forces.  (Loading each step's fields one step ahead was
+// measured slower, 0.244 against 0.237 ms on the 88k-atom box.)
+template <int COUL, bool LJ, bool SWITCH, bool ENERGY, bool DUMP, bool WL>
+__device__ __forceinline__ void sweep64(const NbArgs &a, const SysDev &sd, const PairI2 &I2,
+                                        const PkC &pc, int ik, int lane, unsigned sa,
+                                        ItemSums<COUL> &S) {
+    constexpr bool kFixed = COUL == MDG_COUL_EWALD;  // this kernel's other sums
+    const unsigned lanebit = 1u << lane;
+    u64 FJX = 0ull, FJY = 0ull, FJZ = 0ull, CLJ = 0ull, CC = 0ull;
+    // sa is 2048-byte aligned: cell l ^ t of a block lies at
+    // (sa | l << 4) ^ t << 4
+    const unsigned base = sa | ((unsigned)lane << 4);
+    auto step = [&](unsigned t) {
+        const unsigned ad = base ^ (t << 4);
+        u64 X, Y, Z, Q, Sj = 0ull, E = 0ull, M, J = 0ull;
+        lds2x64(ad, X, Y);
+        lds2x64(ad + 512u, Z, Q);
+        if (LJ && WL) lds2x64(ad + 1024u, Sj, E);
+        if (DUMP) lds2x64(ad + 1536u, M, J);
+        else M = lds64(ad + 1536u);
+        pair_interact2<COUL, LJ, SWITCH, ENERGY, DUMP, WL>(a, sd, I2, pc, ik, lanebit, X, Y, Z, Q,
+                                                          Sj, E, M, J, S.FIX, S.FIY, S.FIZ, FJX,
+                                                          FJY, FJZ, CLJ, CC, S.n_in);
+    };
+#pragma unroll 1
+    for (unsigned t = 0; t < 31u; ++t) {
+        step(t);
+        const unsigned m = t ^ (t + 1u);
+        FJX = shfl_xor2(FJX, m);
+        FJY = shfl_xor2(FJY, m);
+        FJZ = shfl_xor2(FJZ, m);
+    }
+    step(31u);
+    if (!DUMP) {
+        float ja, jb, f[3][2];
+        unpk2(lds64(sa + ((unsigned)(lane ^ 31) << 4) + 1544u), ja, jb);
+        unpk2(FJX, f[0][0], f[0][1]);
+        unpk2(FJY, f[1][0], f[1][1]);
+        unpk2(FJZ, f[2][0], f[2][1]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int jk = __float_as_int(h ? jb : ja);
+            if (jk < 0) continue;
+            if (!(fabsf(f[0][h]) < kFixLimit && fabsf(f[1][h]) < kFixLimit &&
+                  fabsf(f[2][h]) < kFixLimit))
+                raise_status(a.status, MDG_ERR_OVERFLOW);
+            fix_red(&a.f[jk], to_fix(f[0][h]));
+            fix_red(&a.f[a.n_pad + jk], to_fix(f[1][h]));
+            fix_red(&a.f[2 * a.n_pad + jk], to_fix(f[2][h]));
+        }
+    }
+    if constexpr (kFixed) {
+        if (!DUMP && S.per_chunk) S.end_chain(a);
+    }
+    if (ENERGY) {
+        float p0, p1, q0, q1;
+        unpk2(CLJ, p0, p1);
+        unpk2(CC, q0, q1);
+        if constexpr (kFixed) {
+            const float el = p0 + p1, ec = q0 + q1;
+            if (!(fabsf(el) < kFixLimit && fabsf(ec) < kFixLimit))
+                raise_status(a.status, MDG_ERR_OVERFLOW);
+            S.e_lj += to_fix(el);
+            S.e_c += to_fix(ec);
+        } else {
+            S.e_lj += (double)p0 + (double)p1;
+            S.e_c += (double)q0 + (double)q1;
+        }
+    }
+}
+
+// work items of a cluster of system sd
+__device__ __forceinline__ int item_parts(const NbArgs &a, const SysDev &sd) {
+    return a.by_size ? min(nb_default_parts(sd.n_atoms), a.split) : a.split;
+}
+
+// Candidate clusters of i-cluster I for work item `part` (of n_parts): every
 // (J, periodic image) whose bounding box lies within rc of I's box, offered
-// to candidate(J, image code) in ballot order.  Work item `part` scans
-// batches part, part + split, ... of 32 clusters, so the split warps of one
-// i-cluster share its neighbourhood without talking to each other.
-// Balanced half shell: the cluster pair {I, J} (I != J) belongs to I when
-// I < J and I + J is odd, or when I > J and I + J is even -- every cluster
+// to candidate(J, image code) in ballot order (scan_candidates_one ends with
+// candidate(-1, 0)).
+// Work item `part` scans batches part, part + n_parts, ... of 32 clusters, so the
+// warps of one i-cluster share its neighbourhood without talking to each
+// other.  Balanced half shell: the cluster pair {I, J} (I != J) belongs to I
+// when I < J and I + J is odd, or when I > J and I + J is even -- every cluster
 // owns about half of its neighbours whatever its index; J == I is kept and
-// split by the lane mask.  Periodic images: the nearest image of J's box
-// centre, or all 27 when a box pair spans half the box.
+// split by the lane mask.
+// candidate() is inlined, sweeps and all.  Two forms of the search, the same
+// candidates in the same order: scan_candidates calls it from five places (each
+// search's plain and many-image loops), scan_candidates_one from a single one.
+// One system: all items run the same few loops, and the first is 4 % faster
+// (88k atoms).  A batch runs every loop at once: with five copies it spent more
+// on instruction fetch than on anything else (no_instruction 2.5 of 9.1 stalled
+// warps per issue; 40 boxes of 1.5k-12k atoms 378 against 333 us, with energies
+// 517 against 424).
 template <bool ENERGY, typename Cand>
 __device__ __forceinline__ void scan_candidates(const NbArgs &a, const int I, const int part,
-                                                const SysDev &sd, const float4 cI,
-                                                const float4 hI, Cand &&candidate,
-                                                unsigned &n_cand) {
+                                                const int n_parts, const SysDev &sd,
+                                                const float4 cI, const float4 hI,
+                                                Cand &&candidate, unsigned &n_cand) {
     const float L[3] = {sd.L[0], sd.L[1], sd.L[2]};
     const float invL[3] = {sd.invL[0], sd.invL[1], sd.invL[2]};
     const int cl_lo = sd.cl_off, cl_hi = sd.cl_off + sd.cl_cap;
@@ -529,7 +690,7 @@ __device__ __forceinline__ void scan_candidates(const NbArgs &a, const int I, co
                 if (lane >= o) incl += t;
             }
             const int total = __shfl_sync(kFull, incl, 31);
-            for (int v0 = part * 32; v0 < total; v0 += a.split * 32) {
+            for (int v0 = part * 32; v0 < total; v0 += n_parts * 32) {
                 const int v = v0 + lane;
                 int lo = 0, hi = 31;  // first lane whose inclusive count exceeds v
 #pragma unroll
@@ -582,7 +743,7 @@ __device__ __forceinline__ void scan_candidates(const NbArgs &a, const int I, co
     } else {
         // full scan of the system's clusters: work item `part` takes batches
         // part, part + split, ... of 32 clusters
-        for (int J0 = cl_lo + part * 32; J0 < cl_hi; J0 += a.split * 32) {
+        for (int J0 = cl_lo + part * 32; J0 < cl_hi; J0 += n_parts * 32) {
             const int J = J0 + lane;
             bool valid = J < cl_hi && owned(J);
             float4 cJ = make_float4(kFarAway, kFarAway, kFarAway, 0.f),
@@ -632,10 +793,181 @@ __device__ __forceinline__ void scan_candidates(const NbArgs &a, const int I, co
     }
 }
 
+template <bool ENERGY, typename Cand>
+__device__ __forceinline__ void scan_candidates_one(const NbArgs &a, const int I, const int part,
+                                                    const int n_parts, const SysDev &sd,
+                                                    const float4 cI, const float4 hI,
+                                                    Cand &&candidate, unsigned &n_cand) {
+    const float L[3] = {sd.L[0], sd.L[1], sd.L[2]};
+    const float invL[3] = {sd.invL[0], sd.invL[1], sd.invL[2]};
+    const int lane = threadIdx.x & 31;
+    // Column mode (systems whose columns span at least 2R+1 in x and y):
+    // candidates come only from the (2R+1)^2 columns around I's column, R =
+    // the column reach of rc plus twice the largest distance any cluster box
+    // has moved out of its column since the last re-sort.  Each column is a
+    // contiguous run of clusters; the runs of 32 columns at a time are
+    // concatenated into one virtual list (warp scan of the run lengths) walked
+    // 32 at a time.  Otherwise: a full scan of the system's clusters.
+    int R = 0, cx = 0, cy = 0;
+    bool colmode = sd.col_mode != 0;
+    if (colmode) {
+        const float ov = a.overhang[a.cl_sys[I]];
+        const float aw = fminf(L[0] / (float)sd.ncx, L[1] / (float)sd.ncy);
+        R = (int)floorf((a.rc + 2.f * ov) / aw) + 1;
+        colmode = 2 * R + 1 <= min(sd.ncx, sd.ncy);
+        const int pk = a.col_xy[a.cl_col[I]];
+        cx = pk >> 16;
+        cy = pk & 0xffff;
+    }
+    const int side = 2 * R + 1, ncn = colmode ? side * side : 1;
+    // the list being walked: next entry v0, its length; next 32 columns cb
+    int v0 = 0, total = 0, cb = 0;
+    int incl = 0, cnt = 0, start = sd.cl_off, shc = 4;  // shc: (sx + 1) * 3 + (sy + 1)
+    // the current batch: this lane's cluster and the images it hits (bit =
+    // code), and the images left to offer (bit 31: one pass, each lane its own)
+    int J = 0, zshift = 0;
+    unsigned im = 0u, left = 0u;
+    constexpr unsigned kOwn = 1u << 31;
+    for (;;) {
+        bool done = false;
+        if (left == 0u) {  // the next batch
+            while (v0 >= total && cb < ncn) {
+                if (colmode) {
+                    const int c = cb + lane;
+                    cnt = 0;
+                    start = 0;
+                    if (c < ncn) {
+                        int x2 = cx + c / side - R, y2 = cy + c % side - R;
+                        const int sx = x2 < 0 ? -1 : (x2 >= sd.ncx ? 1 : 0);
+                        const int sy = y2 < 0 ? -1 : (y2 >= sd.ncy ? 1 : 0);
+                        x2 -= sx * sd.ncx;
+                        y2 -= sy * sd.ncy;
+                        const int gc = sd.col_off + a.col_rank[sd.col_off + x2 * sd.ncy + y2];
+                        start = sd.cl_off + a.col_cl_start[gc] - a.col_cl_start[sd.col_off];
+                        cnt = a.col_ncl[gc];
+                        shc = (sx + 1) * 3 + (sy + 1);
+                    }
+                    incl = cnt;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int t = __shfl_up_sync(kFull, incl, o);
+                        if (lane >= o) incl += t;
+                    }
+                    total = __shfl_sync(kFull, incl, 31);
+                } else {
+                    total = sd.cl_cap;
+                }
+                v0 = part * 32;
+                cb += 32;
+            }
+            done = v0 >= total;
+            left = kOwn;
+            im = 0u;
+            if (!done) {
+                const int v = v0 + lane;
+                v0 += n_parts * 32;
+                int s_shc = 4;
+                J = sd.cl_off + v;
+                if (colmode) {
+                    int lo = 0, hi = 31;  // first lane whose inclusive count exceeds v
+#pragma unroll
+                    for (int it = 0; it < 5; ++it) {
+                        const int mid = (lo + hi) >> 1;
+                        const int t = __shfl_sync(kFull, incl, mid);
+                        if (t > v) hi = mid;
+                        else lo = mid + 1;
+                    }
+                    const int s_incl = __shfl_sync(kFull, incl, lo);
+                    const int s_cnt = __shfl_sync(kFull, cnt, lo);
+                    const int s_start = __shfl_sync(kFull, start, lo);
+                    s_shc = __shfl_sync(kFull, shc, lo);
+                    J = s_start + (v - (s_incl - s_cnt));
+                }
+                bool valid = v < total && (J == I || ((I + J) & 1) == (I < J ? 1 : 0));
+                float4 cJ = make_float4(kFarAway, kFarAway, kFarAway, 0.f),
+                       hJ = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (valid) {
+                    cJ = a.bbox[2 * J];
+                    hJ = a.bbox[2 * J + 1];
+                }
+                valid = valid && cJ.w > 0.f;
+                const float d[3] = {cJ.x - cI.x, cJ.y - cI.y, cJ.z - cI.z};
+                const float h[3] = {hI.x + hJ.x, hI.y + hJ.y, hI.z + hJ.z};
+                auto gap = [&](int k, float n) {  // between the boxes, along one axis
+                    return fmaxf(fabsf(fmaf(n, L[k], d[k])) - h[k], 0.f);
+                };
+                auto nearest = [&](int k) { return fminf(fmaxf(-rintf(d[k] * invL[k]), -1.f), 1.f); };
+                if (colmode) {
+                    // x and y images follow from the column wrap; z takes the
+                    // nearest image of the box centres, or all three when a box
+                    // pair spans half the box height
+                    const float gx = gap(0, (float)(s_shc / 3 - 1)), gy = gap(1, (float)(s_shc % 3 - 1));
+                    const float gxy = fmaf(gx, gx, gy * gy);
+                    const float nz = nearest(2), gz = gap(2, nz);
+                    const int c0 = s_shc * 3;
+                    if (valid && fmaf(gz, gz, gxy) <= a.rc2) im = 1u << (c0 + (int)nz + 1);
+                    const bool multi = valid && (h[2] + a.rc >= 0.5f * L[2]);
+                    if (__any_sync(kFull, multi)) {
+                        for (int zz = 0; zz < 3; ++zz) {
+                            const float g = gap(2, (float)(zz - 1));
+                            if (multi && fmaf(g, g, gxy) <= a.rc2) im |= 1u << (c0 + zz);
+                        }
+                        left = __reduce_or_sync(kFull, im >> c0);  // z images in turn
+                        zshift = c0;
+                    }
+                } else {
+                    float g2 = 0.f;
+                    int code = 0;
+                    bool multi = valid;
+                    bool wide = false;
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {
+                        const float n = nearest(k), g = gap(k, n);
+                        g2 = fmaf(g, g, g2);
+                        code = code * 3 + (int)n + 1;
+                        wide = wide || (h[k] + a.rc >= 0.5f * L[k]);
+                    }
+                    multi = multi && wide;
+                    if (valid && g2 <= a.rc2) im = 1u << code;
+                    if (__any_sync(kFull, multi)) {
+#pragma unroll 1
+                        for (int c = 0; c < 27; ++c) {
+                            float q2 = 0.f;
+                            const float gs[3] = {gap(0, (float)(c / 9 - 1)), gap(1, (float)((c / 3) % 3 - 1)),
+                                                 gap(2, (float)(c % 3 - 1))};
+#pragma unroll
+                            for (int k = 0; k < 3; ++k) q2 = fmaf(gs[k], gs[k], q2);
+                            if (multi && q2 <= a.rc2) im |= 1u << c;
+                        }
+                        left = __reduce_or_sync(kFull, im);
+                    }
+                }
+                if (left == 0u) left = kOwn;
+            }
+        }
+        // the lowest image left, or each lane's own
+        const unsigned bit = left & (0u - left);
+        left &= left - 1u;
+        const int low = __ffs(bit) - 1;
+        const bool hit = bit == kOwn ? im != 0u : (im >> (low + zshift)) & 1u;
+        const int code = bit == kOwn ? __ffs(im) - 1 : low + zshift;
+        // every lane offers one (J, image); the hits go to candidate()
+        unsigned b = __ballot_sync(kFull, hit);
+        if (ENERGY && !done) n_cand += __popc(b);
+        if (done) b = 1u;
+        while (b) {
+            const int src = __ffs(b) - 1;
+            b &= b - 1;
+            candidate(done ? -1 : __shfl_sync(kFull, J, src), __shfl_sync(kFull, code, src));
+        }
+        if (done) break;
+    }
+}
+
 // One work item: part `part` (of a.split) of i-cluster I's pair search.
 // HALF: the warp's two 16-lane halves sweep separate j lists, each holding
 // only the j atoms within rc of its own 16 i atoms' box.
-template <int COUL, bool LJ, bool SWITCH, bool ENERGY, bool DUMP, bool HALF>
+template <int COUL, bool LJ, bool SWITCH, bool ENERGY, bool DUMP, bool HALF, bool ONE>
 __device__ __forceinline__ void nb_item(const NbArgs &a, const int I, const int part,
                                         float4 *s_j) {
     // rings of 64 entries (2 float4 each): L = j atoms with LJ parameters,
@@ -647,6 +979,8 @@ __device__ __forceinline__ void nb_item(const NbArgs &a, const int I, const int 
     // this cluster's system and its box
     const int sid = a.cl_sys[I];
     const SysDev &sd = a.sys[sid];
+    const int n_parts = item_parts(a, sd);
+    if (part >= n_parts) return;
     const float L[3] = {sd.L[0], sd.L[1], sd.L[2]};
     const int lane = threadIdx.x;
     const unsigned lt = (1u << lane) - 1u;
@@ -662,30 +996,10 @@ __device__ __forceinline__ void nb_item(const NbArgs &a, const int I, const int 
     // whole warp: the packed rings, this lane's i atom in both halves, the
     // packed constants and the packed i-force sums (+fr d, negated at the end)
     float *const pringL = (float *)s_j, *const pringQ = (float *)s_j + 2 * kPkChunk;
-    PairI2 I2;
-    I2.X = splat2(xi.x);
-    I2.Y = splat2(xi.y);
-    I2.Z = splat2(xi.z);
-    I2.Q = splat2(xi.w);
-    I2.S = splat2(pi.x);
-    I2.E = splat2(pi.y);
-    PkC pc;
-    pc.one = splat2(1.0f);
-    pc.six = splat2(6.0f);
-    pc.twelve = splat2(12.0f);
-    pc.a1 = splat2(kAsA1);
-    pc.a2 = splat2(kAsA2);
-    pc.a3 = splat2(kAsA3);
-    pc.a4 = splat2(kAsA4);
-    pc.a5 = splat2(kAsA5);
-    pc.fc = splat2(a.ewald_fc);
-    pc.g = splat2(a.sw_g);
-#if MDG_PK_EWALD_ARGS
-    pc.bp = splat2(a.beta_p);
-    pc.negc = splat2(-a.ewald_exp_c);
-#endif
-    unsigned n_in_lane = 0;  // energy variant: this lane's in-cutoff pairs (packed sweep)
-    u64 FIX = 0ull, FIY = 0ull, FIZ = 0ull;
+    const PairI2 I2 = pair_i2(xi, pi);
+    const PkC pc = pk_constants(a);
+    ItemSums<COUL> S;  // whole warp: i forces and energies
+    if constexpr (COUL == MDG_COUL_EWALD) S.per_chunk = ONE && sd.n_atoms < kNbBlockSystem;
     unsigned long long n_eval = 0, n_in = 0;
     // two rings: j atoms with LJ parameters, and charge-only j atoms, whose
     // sweeps skip the LJ arithmetic (two of every three water atoms)
@@ -762,63 +1076,10 @@ __device__ __forceinline__ void nb_item(const NbArgs &a, const int I, const int 
     };
     auto shared_addr = [](const float4 *p) { return (unsigned)__cvta_generic_to_shared(p); };
     auto shared_addr_f = [](const float *p) { return (unsigned)__cvta_generic_to_shared(p); };
-    auto push_j = [&](int jk, float fjx, float fjy, float fjz) {
-        if (jk >= 0 && !DUMP) {
-            if (!(fabsf(fjx) < kFixLimit && fabsf(fjy) < kFixLimit && fabsf(fjz) < kFixLimit))
-                raise_status(a.status, MDG_ERR_OVERFLOW);
-            fix_red(&a.f[jk], to_fix(fjx));
-            fix_red(&a.f[a.n_pad + jk], to_fix(fjy));
-            fix_red(&a.f[2 * a.n_pad + jk], to_fix(fjz));
-        }
-    };
-    // Whole warp: one packed super-chunk (64 j atoms as 32 (A, B) pairs) at
-    // byte address sa, swept in 32 rotation steps: at step t lane l pairs its
-    // i atom with pair l ^ t (both halves at once), the pair's j-force
-    // accumulators travel by butterfly shuffles (mask t ^ (t + 1)), and
-    // after step 31 lane l owns pair l ^ 31's two j forces.  (Loading each
-    // step's fields one step ahead was measured slower, 0.244 against 0.237
-    // ms on the 88k-atom box.)
+    // Whole warp: one packed super-chunk at byte address sa
     auto chunk64 = [&](auto with_lj, unsigned sa) {
         constexpr bool WL = decltype(with_lj)::value;
-        u64 FJX = 0ull, FJY = 0ull, FJZ = 0ull, CLJ = 0ull, CC = 0ull;
-        // sa is 2048-byte aligned: cell l ^ t of a block lies at
-        // (sa | l << 4) ^ t << 4; the last step needs no shuffle
-        const unsigned base = sa | ((unsigned)lane << 4);
-        auto step = [&](unsigned t) {
-            const unsigned ad = base ^ (t << 4);
-            u64 X, Y, Z, Q, S = 0ull, E = 0ull, M, J = 0ull;
-            lds2x64(ad, X, Y);
-            lds2x64(ad + 512u, Z, Q);
-            if (LJ && WL) lds2x64(ad + 1024u, S, E);
-            if (DUMP) lds2x64(ad + 1536u, M, J);
-            else M = lds64(ad + 1536u);
-            pair_interact2<COUL, LJ, SWITCH, ENERGY, DUMP, WL>(a, sd, I2, pc, ik, lanebit, X, Y, Z, Q,
-                                                              S, E, M, J, FIX, FIY, FIZ, FJX,
-                                                              FJY, FJZ, CLJ, CC, n_in_lane);
-        };
-#pragma unroll 1
-        for (unsigned t = 0; t < 31u; ++t) {
-            step(t);
-            const unsigned m = t ^ (t + 1u);
-            FJX = shfl_xor2(FJX, m);
-            FJY = shfl_xor2(FJY, m);
-            FJZ = shfl_xor2(FJZ, m);
-        }
-        step(31u);
-        float ja, jb, xa, xb, ya, yb, za, zb;
-        unpk2(lds64(sa + ((unsigned)(lane ^ 31) << 4) + 1544u), ja, jb);
-        unpk2(FJX, xa, xb);
-        unpk2(FJY, ya, yb);
-        unpk2(FJZ, za, zb);
-        push_j(__float_as_int(ja), xa, ya, za);
-        push_j(__float_as_int(jb), xb, yb, zb);
-        if (ENERGY) {
-            float p0, p1, q0, q1;
-            unpk2(CLJ, p0, p1);
-            unpk2(CC, q0, q1);
-            acc_lj += (double)p0 + (double)p1;
-            acc_c += (double)q0 + (double)q1;
-        }
+        sweep64<COUL, LJ, SWITCH, ENERGY, DUMP, WL>(a, sd, I2, pc, ik, lane, sa, S);
         n_eval += 2048;
         __syncwarp();
     };
@@ -846,7 +1107,7 @@ __device__ __forceinline__ void nb_item(const NbArgs &a, const int I, const int 
 
     // one candidate (J, image) found by the scan: test J's atoms against I's box
     // and append the survivors to this warp's ring (chunk sweeps when full)
-    auto candidate = [&](int J, int code) {
+    auto append = [&](int J, int code) -> bool {
         float sx, sy, sz;
         decode_shift(code, L, sx, sy, sz);
         const int jk = J * kCluster + lane;
@@ -888,7 +1149,7 @@ __device__ __forceinline__ void nb_item(const NbArgs &a, const int I, const int 
             const bool bL = hitB && to_l, bQ = hitB && !to_l && keep_q;
             const unsigned mAL = __ballot_sync(kFull, aL), mAQ = __ballot_sync(kFull, aQ);
             const unsigned mBL = __ballot_sync(kFull, bL), mBQ = __ballot_sync(kFull, bQ);
-            if ((mAL | mAQ | mBL | mBQ) == 0u) return;
+            if ((mAL | mAQ | mBL | mBQ) == 0u) return false;
             if (aL || aQ || bL || bQ) {
                 const unsigned m = excl_mask();
                 if (aL) put_entry(ringL, (jbL + jcL + __popc(mAL & lt)) & (kRing - 1), xj, pj, m, jk);
@@ -904,7 +1165,7 @@ __device__ __forceinline__ void nb_item(const NbArgs &a, const int I, const int 
             // every ring stays below 32 pending entries between candidates
             while (jcL >= 32 || jcL2 >= 32 || (jcL >= 16 && jcL2 >= 16)) sweep16(std::true_type{});
             while (jcQ >= 32 || jcQ2 >= 32 || (jcQ >= 16 && jcQ2 >= 16)) sweep16(std::false_type{});
-            return;
+            return false;
         }
         const float gx = fmaxf(fabsf(xj.x - cI.x) - hI.x, 0.f);
         const float gy = fmaxf(fabsf(xj.y - cI.y) - hI.y, 0.f);
@@ -918,7 +1179,7 @@ __device__ __forceinline__ void nb_item(const NbArgs &a, const int I, const int 
         const bool hitL = hit && to_l;
         const bool hitQ = hit && !to_l && (COUL == MDG_COUL_EWALD || DUMP);
         const unsigned bL = __ballot_sync(kFull, hitL), bQ = __ballot_sync(kFull, hitQ);
-        if ((bL | bQ) == 0u) return;
+        if ((bL | bQ) == 0u) return false;
         if (hitL || hitQ) {
             const unsigned m = excl_mask();
             if (hitL)
@@ -928,6 +1189,38 @@ __device__ __forceinline__ void nb_item(const NbArgs &a, const int I, const int 
         }
         jcL += __popc(bL);
         jcQ += __popc(bQ);
+        return true;
+    };
+    // the partial super-chunks at the end: charge-only slots join the LJ ring
+    // when both fit in one (their LJ terms are zero), then each partial one is
+    // padded with far-away slots up to 64
+    auto fill_up = [&]() {
+        if (jcQ > 0 && jcL + jcQ <= 64) {
+            for (int k = lane; k < jcQ; k += 32)
+                copy_entry_pk(pringQ, (jbQ + k) & (kPkRing - 1), pringL,
+                              (jbL + jcL + k) & (kPkRing - 1));
+            jcL += jcQ;
+            jcQ = 0;
+            __syncwarp();
+        }
+        auto pad = [&](float *ring, int jb, int &jc) {
+            if (jc == 0) return;
+            for (int k = jc + lane; k < 64; k += 32)
+                put_entry_pk(ring, (jb + k) & (kPkRing - 1),
+                             make_float4(kFarAway, kFarAway, kFarAway, 0.f), make_float2(0.f, 0.f),
+                             kFull, -1);
+            jc = 64;
+        };
+        pad(pringL, jbL, jcL);
+        pad(pringQ, jbQ, jcQ);
+    };
+    auto candidate = [&](int J, int code) {
+        if (J >= 0) {
+            if (!append(J, code)) return;
+        } else {
+            if constexpr (!ONE) return;
+            fill_up();
+        }
         __syncwarp();
         // a full super-chunk of a ring is swept; between candidates a ring
         // holds fewer than 64 pending slots (a candidate adds at most 32, so
@@ -945,7 +1238,16 @@ __device__ __forceinline__ void nb_item(const NbArgs &a, const int I, const int 
     };
 
     unsigned n_cand = 0;
-    scan_candidates<ENERGY>(a, I, part, sd, cI, hI, candidate, n_cand);
+    if constexpr (ONE)
+        scan_candidates_one<ENERGY>(a, I, part, n_parts, sd, cI, hI, candidate, n_cand);
+    else
+        scan_candidates<ENERGY>(a, I, part, n_parts, sd, cI, hI, candidate, n_cand);
+    if constexpr (!ONE && !HALF) {
+        fill_up();
+        __syncwarp();
+        if (jcL >= 64) chunk64(std::true_type{}, shared_addr_f(pringL + (jbL >> 6) * kPkChunk));
+        if (jcQ >= 64) chunk64(std::false_type{}, shared_addr_f(pringQ + (jbQ >> 6) * kPkChunk));
+    }
     // The partial last chunks, padded with far-away entries.  When both fit
     // in one chunk the charge-only entries join the LJ chunk (their LJ terms
     // are zero), so an item ends with at most one partial sweep.
@@ -967,40 +1269,29 @@ __device__ __forceinline__ void nb_item(const NbArgs &a, const int I, const int 
         while (jcQ > 0 || jcQ2 > 0) sweep16(std::false_type{});
     }
     if constexpr (!HALF) {
-        // the partial super-chunks: charge-only slots join the LJ ring when
-        // both fit in one (their LJ terms are zero), then each partial one is
-        // padded with far-away slots up to 64 and swept
-        if (jcQ > 0 && jcL + jcQ <= 64) {
-            for (int k = lane; k < jcQ; k += 32)
-                copy_entry_pk(pringQ, (jbQ + k) & (kPkRing - 1), pringL,
-                              (jbL + jcL + k) & (kPkRing - 1));
-            jcL += jcQ;
-            jcQ = 0;
-            __syncwarp();
+        if constexpr (COUL != MDG_COUL_EWALD) {
+            float a0, a1, b0, b1, c0, c1;
+            unpk2(S.FIX, a0, a1);
+            unpk2(S.FIY, b0, b1);
+            unpk2(S.FIZ, c0, c1);
+            fix -= a0 + a1;
+            fiy -= b0 + b1;
+            fiz -= c0 + c1;
         }
-        auto finish = [&](auto with_lj, float *ring, int jb, int jc) {
-            if (jc == 0) return;
-            for (int k = jc + lane; k < 64; k += 32)
-                put_entry_pk(ring, (jb + k) & (kPkRing - 1),
-                             make_float4(kFarAway, kFarAway, kFarAway, 0.f), make_float2(0.f, 0.f),
-                             kFull, -1);
-            __syncwarp();
-            chunk64(with_lj, shared_addr_f(ring + (jb >> 6) * kPkChunk));
-        };
-        finish(std::true_type{}, pringL, jbL, jcL);
-        finish(std::false_type{}, pringQ, jbQ, jcQ);
-        float a0, a1, b0, b1, c0, c1;
-        unpk2(FIX, a0, a1);
-        unpk2(FIY, b0, b1);
-        unpk2(FIZ, c0, c1);
-        fix -= a0 + a1;
-        fiy -= b0 + b1;
-        fiz -= c0 + c1;
-        if (ENERGY) n_in += __reduce_add_sync(kFull, n_in_lane);
+        if (ENERGY) {
+            n_in += __reduce_add_sync(kFull, S.n_in);
+            if constexpr (COUL != MDG_COUL_EWALD) {
+                acc_lj = S.e_lj;
+                acc_c = S.e_c;
+            }
+        }
     }
 
     // ---- this work item's share of the i forces and energies -------------
-    if (!DUMP && i_real) {
+    if constexpr (!DUMP && !HALF && COUL == MDG_COUL_EWALD) {
+        if (!S.per_chunk) S.end_chain(a);
+        if (i_real) S.push_i(a, ik);
+    } else if (!DUMP && i_real) {
         if (!(fabsf(fix) < kFixLimit && fabsf(fiy) < kFixLimit && fabsf(fiz) < kFixLimit))
             raise_status(a.status, MDG_ERR_OVERFLOW);
         fix_red(&a.f[ik], to_fix(fix));
@@ -1008,17 +1299,202 @@ __device__ __forceinline__ void nb_item(const NbArgs &a, const int I, const int 
         fix_red(&a.f[2 * a.n_pad + ik], to_fix(fiz));
     }
     if (ENERGY) {
-        const double el = warp_sum_d(acc_lj), ee = warp_sum_d(acc_c);
-        if (lane == 0) {
-            if (!(fabs(el) < kFixLimit && fabs(ee) < kFixLimit))
+        long long el, ee;  // fixed point
+        if constexpr (!HALF && COUL == MDG_COUL_EWALD) {
+            el = warp_sum_ll(S.e_lj);
+            ee = warp_sum_ll(S.e_c);
+        } else {
+            const double dl = warp_sum_d(acc_lj), dc = warp_sum_d(acc_c);
+            if (lane == 0 && !(fabs(dl) < kFixLimit && fabs(dc) < kFixLimit))
                 raise_status(a.status, MDG_ERR_OVERFLOW);
+            el = to_fix_d(dl);
+            ee = to_fix_d(dc);
+        }
+        if (lane == 0) {
             long long *es = a.energy + sid * kEnergySlots;
-            fix_red((unsigned long long *)&es[MDG_TERM_LJ], to_fix_d(el));
-            fix_red((unsigned long long *)&es[MDG_TERM_COUL_REAL], to_fix_d(ee));
+            fix_red((unsigned long long *)&es[MDG_TERM_LJ], el);
+            fix_red((unsigned long long *)&es[MDG_TERM_COUL_REAL], ee);
             atomicAdd(&a.stats[0], n_eval);
             atomicAdd(&a.stats[1], n_in);
             atomicAdd(&a.stats[2], (unsigned long long)n_cand);
             if (part == 0) atomicAdd(&a.stats[3], 1ull);
+        }
+    }
+}
+
+// ---- block form --------------------------------------------------------------
+// A whole-warp item taken by W warps (2, 4 or 8) of one block, for systems
+// whose items alone leave most of the GPU's warp slots empty.  Every warp runs
+// the candidate scan; of each W candidates in scan order warp w loads and tests
+// the w-th, and the survivors are appended to the two rings in candidate order
+// (each warp's place from the counts of the warps before it, one block barrier
+// a round).  When a ring could not take another round, its full super-chunks
+// are swept, one per warp in turn.  The rings therefore hold the super-chunks
+// that one warp would have built, and the sums across super-chunks are fixed
+// point: the forces and energies are the one-warp form's bit for bit.
+// Bound by latency: a round is one dependent chain of loads (about 1000
+// cycles), a sweep 32 dependent steps, both spread over W warps here.
+// super-chunks per ring: room for one round (32 W slots) above the partial one,
+// and W warps' worth of sweeps between rounds
+__host__ __device__ constexpr int nb_block_chunks(int warps) { return warps == 8 ? 8 : warps == 4 ? 6 : 5; }
+
+template <int COUL, bool LJ, bool SWITCH, bool ENERGY>
+__global__ void __launch_bounds__(256, 2) k_nonbonded_block(NbArgs a) {
+    extern __shared__ __align__(2048) float s_rings[];
+    __shared__ int2 s_cnt[2][8];
+    const int W = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nc = nb_block_chunks(W), cap = nc * 64;
+    float *const ringL = s_rings, *const ringQ = s_rings + nc * kPkChunk;
+    const int I = blockIdx.x / a.split, part = blockIdx.x % a.split;
+    const float4 cI = a.bbox[2 * I], hI = a.bbox[2 * I + 1];
+    if (cI.w == 0.f) return;  // all-padding cluster: the whole block leaves
+    const int sid = a.cl_sys[I];
+    const SysDev &sd = a.sys[sid];
+    const int n_parts = item_parts(a, sd);
+    if (part >= n_parts) return;
+    const float L[3] = {sd.L[0], sd.L[1], sd.L[2]};
+    const unsigned lt = (1u << lane) - 1u;
+    const int ik = I * kCluster + lane, ilo = I * kCluster;
+    const float4 xi = a.xq[ik];
+    const PairI2 I2 = pair_i2(xi, a.prm[ik]);
+    const PkC pc = pk_constants(a);
+    const int2 rI = a.prange[I];
+    ItemSums<COUL> S;
+    unsigned long long n_eval = 0;
+    // first chunk and pending slots of each ring, the same in every warp
+    int bL = 0, jcL = 0, bQ = 0, jcQ = 0, par = 0;
+    auto slot = [&](int b, int k) {  // ring slot of pending entry k
+        const int p = b * 64 + k;
+        return p >= cap ? p - cap : p;
+    };
+    auto addr = [&](float *ring, int b, int k) {
+        const int c = b + k >= nc ? b + k - nc : b + k;
+        return (unsigned)__cvta_generic_to_shared(ring + c * kPkChunk);
+    };
+    // Sweeps of the full super-chunks, one per warp in turn.  At the end of the
+    // scan a second pass takes the partial ones, merged and padded as the
+    // one-warp form does.
+    auto sweep_full = [&](bool last) {
+        for (int pass = 0; pass <= (last ? 1 : 0); ++pass) {
+            if (pass == 1) {
+                if (jcQ > 0 && jcL + jcQ <= 64) {
+                    if (w == 0)
+                        for (int k = lane; k < jcQ; k += 32)
+                            copy_entry_pk(ringQ, slot(bQ, k), ringL, slot(bL, jcL + k));
+                    jcL += jcQ;
+                    jcQ = 0;
+                }
+                auto pad = [&](float *ring, int b, int &jc, int warp) {
+                    if (jc == 0) return;
+                    if (w == warp)
+                        for (int k = jc + lane; k < 64; k += 32)
+                            put_entry_pk(ring, slot(b, k),
+                                         make_float4(kFarAway, kFarAway, kFarAway, 0.f),
+                                         make_float2(0.f, 0.f), kFull, -1);
+                    jc = 64;
+                };
+                pad(ringL, bL, jcL, 0);
+                pad(ringQ, bQ, jcQ, 1);
+            }
+            __syncthreads();  // every entry is written
+            const int nL = jcL >> 6, nQ = jcQ >> 6;
+            for (int t = w; t < nL + nQ; t += W) {
+                const bool lj = t < nL;
+                const unsigned sa = lj ? addr(ringL, bL, t) : addr(ringQ, bQ, t - nL);
+                if (lj) sweep64<COUL, LJ, SWITCH, ENERGY, false, true>(a, sd, I2, pc, ik, lane, sa, S);
+                else sweep64<COUL, LJ, SWITCH, ENERGY, false, false>(a, sd, I2, pc, ik, lane, sa, S);
+                n_eval += 2048;
+            }
+            bL = bL + nL >= nc ? bL + nL - nc : bL + nL;
+            bQ = bQ + nQ >= nc ? bQ + nQ - nc : bQ + nQ;
+            jcL &= 63;
+            jcQ &= 63;
+            __syncthreads();  // the swept chunks may be overwritten
+        }
+    };
+    int nh = 0, myJ = -1, mycode = 0;  // candidates of this round; this warp's
+    auto candidate = [&](int J, int code) {
+        const bool last = J < 0;
+        if (!last) {
+            if (nh == w) {
+                myJ = J;
+                mycode = code;
+            }
+            if (++nh < W) return;
+        }
+        float4 xj = make_float4(0.f, 0.f, 0.f, 0.f);
+        float2 pj = make_float2(0.f, 0.f);
+        bool hitL = false, hitQ = false;
+        const int jk = myJ * kCluster + lane;
+        if (myJ >= 0) {
+            float sx, sy, sz;
+            decode_shift(mycode, L, sx, sy, sz);
+            xj = a.xq[jk];
+            pj = a.prm[jk];
+            xj.x += sx;
+            xj.y += sy;
+            xj.z += sz;
+            const float gx = fmaxf(fabsf(xj.x - cI.x) - hI.x, 0.f);
+            const float gy = fmaxf(fabsf(xj.y - cI.y) - hI.y, 0.f);
+            const float gz = fmaxf(fabsf(xj.z - cI.z) - hI.z, 0.f);
+            const bool hit = fmaf(gx, gx, fmaf(gy, gy, gz * gz)) <= a.rc2;
+            const bool to_l = !a.split_rings || (LJ && pj.y != 0.f);
+            hitL = hit && to_l;
+            hitQ = hit && !to_l;
+        }
+        const unsigned mL = __ballot_sync(kFull, hitL), mQ = __ballot_sync(kFull, hitQ);
+        if (lane == 0) s_cnt[par][w] = make_int2(__popc(mL), __popc(mQ));
+        __syncthreads();
+        int oL = jcL, oQ = jcQ, tL = 0, tQ = 0;
+        for (int k = 0; k < W; ++k) {
+            const int2 c = s_cnt[par][k];
+            if (k < w) {
+                oL += c.x;
+                oQ += c.y;
+            }
+            tL += c.x;
+            tQ += c.y;
+        }
+        // the next round writes the other half of s_cnt; this half is written
+        // again only after that round's barrier, which follows these reads
+        par ^= 1;
+        if (hitL || hitQ) {
+            unsigned m = 0u;  // exclusion mask of the i lanes for this j atom
+            if (myJ == I) m = kFull << lane;  // half shell inside the cluster
+            if (rI.y >= myJ * kCluster && rI.x < (myJ + 1) * kCluster)
+                for (int k = 0; k < a.pw; ++k) {
+                    const int p = a.partners[(size_t)jk * a.pw + k];
+                    const int pk = (p & 0x3fffffff) - ilo;
+                    if (p >= 0 && pk >= 0 && pk < kCluster) m |= 1u << pk;
+                }
+            if (hitL) put_entry_pk(ringL, slot(bL, oL + __popc(mL & lt)), xj, pj, m, jk);
+            else put_entry_pk(ringQ, slot(bQ, oQ + __popc(mQ & lt)), xj, pj, m, jk);
+        }
+        jcL += tL;
+        jcQ += tQ;
+        nh = 0;
+        myJ = -1;
+        // a round's entries reach another warp's copy or padding only behind
+        // a barrier (the first pass of the last call has one)
+        if (last || max(jcL, jcQ) > cap - 32 * W) sweep_full(last);
+    };
+    unsigned n_cand = 0;
+    scan_candidates_one<ENERGY>(a, I, part, n_parts, sd, cI, hI, candidate, n_cand);
+
+    if (n_eval > 0 && xi.x < 0.5f * kFarAway) S.push_i(a, ik);
+    if (ENERGY) {
+        const unsigned n_in = __reduce_add_sync(kFull, S.n_in);
+        const long long el = warp_sum_ll(S.e_lj), ec = warp_sum_ll(S.e_c);
+        if (lane == 0) {
+            long long *es = a.energy + sid * kEnergySlots;
+            fix_red((unsigned long long *)&es[MDG_TERM_LJ], el);
+            fix_red((unsigned long long *)&es[MDG_TERM_COUL_REAL], ec);
+            atomicAdd(&a.stats[0], n_eval);
+            atomicAdd(&a.stats[1], (unsigned long long)n_in);
+            if (w == 0) {
+                atomicAdd(&a.stats[2], (unsigned long long)n_cand);
+                if (part == 0) atomicAdd(&a.stats[3], 1ull);
+            }
         }
     }
 }
@@ -1046,6 +1522,8 @@ __device__ __forceinline__ void nb_item_q(const NbArgs &a, const int I, const in
     if (cI.w == 0.f) return;  // all-padding cluster
     const int sid = a.cl_sys[I];
     const SysDev &sd = a.sys[sid];
+    const int n_parts = item_parts(a, sd);
+    if (part >= n_parts) return;
     const float L[3] = {sd.L[0], sd.L[1], sd.L[2]};
     const int lane = threadIdx.x;
     const int grp = lane >> 3, li = lane & 7;
@@ -1223,7 +1701,7 @@ __device__ __forceinline__ void nb_item_q(const NbArgs &a, const int I, const in
     };
 
     unsigned n_cand = 0;
-    scan_candidates<ENERGY>(a, I, part, sd, cI, hI, candidate, n_cand);
+    scan_candidates<ENERGY>(a, I, part, n_parts, sd, cI, hI, candidate, n_cand);
     drain(true);
 
     if (!DUMP && i_real) {
@@ -1292,7 +1770,7 @@ __global__ void __launch_bounds__(32, ENERGY ? 12 : 13) k_nonbonded_q(NbArgs a) 
 #ifndef MDG_NB_MIN_BLOCKS_HALF
 #define MDG_NB_MIN_BLOCKS_HALF 20
 #endif
-template <int COUL, bool LJ, bool SWITCH, bool ENERGY, bool DUMP, bool HALF>
+template <int COUL, bool LJ, bool SWITCH, bool ENERGY, bool DUMP, bool HALF, bool ONE>
 __global__ void __launch_bounds__(32, ENERGY ? (HALF ? 16 : MDG_NB_MIN_BLOCKS_ENERGY)
                                              : (HALF ? MDG_NB_MIN_BLOCKS_HALF : MDG_NB_MIN_BLOCKS))
     k_nonbonded(NbArgs a) {
@@ -1301,7 +1779,7 @@ __global__ void __launch_bounds__(32, ENERGY ? (HALF ? 16 : MDG_NB_MIN_BLOCKS_EN
     // bytes, each 32-entry chunk on a 1024-byte boundary
     __shared__ __align__(1024) float4 s_j[8 * kRing];
     if (!a.persistent) {
-        nb_item<COUL, LJ, SWITCH, ENERGY, DUMP, HALF>(a, blockIdx.x / a.split, blockIdx.x % a.split,
+        nb_item<COUL, LJ, SWITCH, ENERGY, DUMP, HALF, ONE>(a, blockIdx.x / a.split, blockIdx.x % a.split,
                                                 s_j);
         return;
     }
@@ -1313,52 +1791,52 @@ __global__ void __launch_bounds__(32, ENERGY ? (HALF ? 16 : MDG_NB_MIN_BLOCKS_EN
         const int end = min(base + a.grab, a.n_items);
         for (int item = base; item < end; ++item) {
             __syncwarp();  // the previous item's ring reads are done
-            nb_item<COUL, LJ, SWITCH, ENERGY, DUMP, HALF>(a, item / a.split, item % a.split, s_j);
+            nb_item<COUL, LJ, SWITCH, ENERGY, DUMP, HALF, ONE>(a, item / a.split, item % a.split, s_j);
         }
     }
 }
 
-template <int COUL, bool LJ, bool SW, bool HALF>
+template <int COUL, bool LJ, bool SW, bool HALF, bool ONE>
 cudaError_t dispatch_nb(mdg_system *s, const NbArgs &a, int energy, int dump) {
     dim3 grid(a.persistent ? s->nb_persistent_ctas : a.n_items), block(32);
     if (a.persistent && cudaMemsetAsync(a.queue, 0, sizeof(int), s->stream) != cudaSuccess)
         return cudaGetLastError();
     if (dump) {
-        if constexpr (COUL == MDG_COUL_EWALD && LJ && !SW)
-            k_nonbonded<COUL, LJ, SW, false, true, HALF><<<grid, block, 0, s->stream>>>(a);
+        if constexpr (COUL == MDG_COUL_EWALD && LJ && !SW && !ONE)
+            k_nonbonded<COUL, LJ, SW, false, true, HALF, ONE><<<grid, block, 0, s->stream>>>(a);
     } else if (energy)
-        k_nonbonded<COUL, LJ, SW, true, false, HALF><<<grid, block, 0, s->stream>>>(a);
+        k_nonbonded<COUL, LJ, SW, true, false, HALF, ONE><<<grid, block, 0, s->stream>>>(a);
     else {
 #if MDG_NB_CARVEOUT
         // the shared-memory carveout at its maximum, so that shared memory
         // does not cap the resident CTAs below the register budget's count
         static bool carveout_set = false;
         if (!carveout_set) {
-            cudaFuncSetAttribute(k_nonbonded<COUL, LJ, SW, false, false, HALF>,
+            cudaFuncSetAttribute(k_nonbonded<COUL, LJ, SW, false, false, HALF, ONE>,
                                  cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared);
             carveout_set = true;
         }
 #endif
-        k_nonbonded<COUL, LJ, SW, false, false, HALF><<<grid, block, 0, s->stream>>>(a);
+        k_nonbonded<COUL, LJ, SW, false, false, HALF, ONE><<<grid, block, 0, s->stream>>>(a);
     }
     return cudaGetLastError();
 }
 
 // every (Coulomb, LJ, switch) combination the library launches, for one HALF
-template <bool HALF>
+template <bool HALF, bool ONE = false>
 cudaError_t dispatch_shape(mdg_system *s, const NbArgs &a, int coul_tile, bool want_lj, bool sw,
                            int energy, int dump) {
     // the pair-set dump decides pairs by the reference's test alone, whatever
     // the terms: one instantiation serves every configuration
-    if (dump) return dispatch_nb<MDG_COUL_EWALD, true, false, HALF>(s, a, 0, 1);
+    if (dump) return dispatch_nb<MDG_COUL_EWALD, true, false, HALF, ONE>(s, a, 0, 1);
     if (coul_tile == MDG_COUL_EWALD && !want_lj)
-        return dispatch_nb<MDG_COUL_EWALD, false, false, HALF>(s, a, energy, dump);
+        return dispatch_nb<MDG_COUL_EWALD, false, false, HALF, ONE>(s, a, energy, dump);
     if (coul_tile == MDG_COUL_EWALD)
-        return sw ? dispatch_nb<MDG_COUL_EWALD, true, true, HALF>(s, a, energy, dump)
-                  : dispatch_nb<MDG_COUL_EWALD, true, false, HALF>(s, a, energy, dump);
-    return sw ? dispatch_nb<MDG_COUL_NONE, true, true, HALF>(s, a, energy, dump)
-              : dispatch_nb<MDG_COUL_NONE, true, false, HALF>(s, a, energy, dump);
+        return sw ? dispatch_nb<MDG_COUL_EWALD, true, true, HALF, ONE>(s, a, energy, dump)
+                  : dispatch_nb<MDG_COUL_EWALD, true, false, HALF, ONE>(s, a, energy, dump);
+    return sw ? dispatch_nb<MDG_COUL_NONE, true, true, HALF, ONE>(s, a, energy, dump)
+              : dispatch_nb<MDG_COUL_NONE, true, false, HALF, ONE>(s, a, energy, dump);
 }
 
 }  // namespace
