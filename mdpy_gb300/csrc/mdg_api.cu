@@ -74,14 +74,21 @@ void drop_one(Graph &g) {
     if (g.exec) cudaGraphExecDestroy(g.exec);
     g.exec = nullptr;
     g.steps = 0;
+    g.uses = 0;
 }
 
-void drop_graph(mdg_system *s) {
+void drop_step_graphs(mdg_system *s) {
     drop_one(s->graph);
+    s->chunk_uses = 0;
     for (auto &plane : s->graph_step)
         for (auto &row : plane)
             for (Graph &g : row) drop_one(g);
-    for (Graph &g : s->graph_eval) drop_one(g);
+}
+
+void drop_graph(mdg_system *s) {
+    drop_step_graphs(s);
+    for (auto &row : s->graph_eval)
+        for (Graph &g : row) drop_one(g);
 }
 
 int validate_box(const double *box, double cutoff) {
@@ -153,12 +160,36 @@ int decode_status(mdg_system *s, int st) {
     return MDG_OK;
 }
 
-int read_status(mdg_system *s) {
-    int st = 0;
-    CK(cudaMemcpyAsync(&st, s->status, sizeof(int), cudaMemcpyDeviceToHost, s->stream),
+// The pinned staging words: the energy words of every system, the status word
+// (its low half) and one more.
+size_t stage_words(const mdg_system *s) { return (size_t)kEnergySlots * s->n_sys; }
+
+int stage_ready(mdg_system *s) {
+    if (!s->host_stage)
+        CK(cudaMallocHost((void **)&s->host_stage, sizeof(long long) * (stage_words(s) + 2)),
+           "pinned staging");
+    return MDG_OK;
+}
+
+// A read that ends with one synchronisation: the status word is copied beside
+// what is read (enqueue_status), and decoded after it (finish_status).
+int enqueue_status(mdg_system *s) {
+    const int rc = stage_ready(s);
+    if (rc) return rc;
+    CK(cudaMemcpyAsync(s->host_stage + stage_words(s), s->status, sizeof(int),
+                       cudaMemcpyDeviceToHost, s->stream),
        "status read");
+    return MDG_OK;
+}
+
+int finish_status(mdg_system *s) {
     CK(cudaStreamSynchronize(s->stream), "synchronize");
-    return decode_status(s, st);
+    return decode_status(s, (int)(s->host_stage[stage_words(s)] & 0xffffffffll));
+}
+
+int read_status(mdg_system *s) {
+    const int rc = enqueue_status(s);
+    return rc ? rc : finish_status(s);
 }
 
 int evaluate(mdg_system *s, unsigned mask, int energy) {
@@ -299,14 +330,13 @@ int capture_steps(mdg_system *s, Graph &g, int nsteps, int resort, unsigned mask
     return MDG_OK;
 }
 
-// The force evaluation an integration starts with when the forces are not
-// valid (new positions): captured once per re-sort flag and replayed.
-int capture_eval(mdg_system *s, Graph &g, int resort, unsigned mask) {
+// One force evaluation, captured.
+int capture_eval(mdg_system *s, Graph &g, int resort, unsigned mask, int energy) {
     const long long saved = s->launches;
     const int saved_need = s->need_reorder, saved_since = s->steps_since_reorder;
     s->need_reorder = resort ? 1 : 0;
     CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal), "capture");
-    const int crc = evaluate(s, mask, 0);
+    const int crc = evaluate(s, mask, energy);
     cudaGraph_t graph = nullptr;
     cudaError_t ce = cudaStreamEndCapture(s->stream, &graph);
     s->need_reorder = saved_need;
@@ -326,6 +356,34 @@ int capture_eval(mdg_system *s, Graph &g, int resort, unsigned mask) {
     }
     g.steps = (int)per;
     g.mask = mask;
+    return MDG_OK;
+}
+
+// A force evaluation of the complete terms in `mask`: about 20 launches (30 with
+// a re-sort) of a few microseconds of host time each, so one that comes up again
+// is captured at its third run and replayed from then on (a capture costs about
+// what four eager runs do); always when `now`.
+int run_evaluation(mdg_system *s, unsigned mask, int energy, bool now) {
+    const int resort = s->need_reorder ? 1 : 0;
+    Graph &g = s->graph_eval[energy ? 1 : 0][resort];
+    if (g.mask != mask) {
+        drop_one(g);
+        g.mask = mask;
+    }
+    if (!g.exec && !now && g.uses < 2) {
+        g.uses += 1;
+        return evaluate(s, mask, energy);
+    }
+    if (!g.exec) {
+        const int rc = capture_eval(s, g, resort, mask, energy);
+        if (rc) return rc;
+    }
+    CK(cudaGraphLaunch(g.exec, s->stream), "graph launch");
+    s->launches += g.steps;
+    if (resort) {
+        s->need_reorder = 0;
+        s->steps_since_reorder = 0;
+    }
     return MDG_OK;
 }
 
@@ -947,6 +1005,7 @@ MDG_API int mdg_get_positions(mdg_system *s, double *x, int where) {
     int rc = check_sys(s);
     if (rc) return rc;
     if (!x) return fail(MDG_ERR_INVALID, "output pointer is null");
+    if ((rc = enqueue_status(s))) return rc;
     if (where == MDG_DEVICE) {
         CK(launch_positions_out(s, x), "positions out");
     } else {
@@ -955,8 +1014,7 @@ MDG_API int mdg_get_positions(mdg_system *s, double *x, int where) {
                            s->stream),
            "copy");
     }
-    CK(cudaStreamSynchronize(s->stream), "synchronize");
-    return read_status(s);
+    return finish_status(s);
 }
 
 MDG_API int mdg_get_velocities(mdg_system *s, double *v, int where) {
@@ -977,7 +1035,7 @@ MDG_API int mdg_compute_forces(mdg_system *s, unsigned mask) {
     mask &= MDG_MASK_ALL;
     rc = ready_for_forces(s, mask);
     if (rc) return rc;
-    rc = evaluate(s, mask, 1);
+    rc = run_evaluation(s, mask, 1, false);
     if (rc) return rc;
     s->forces_valid = 1;
     s->forces_mask = mask;
@@ -991,28 +1049,28 @@ MDG_API int mdg_get_forces(mdg_system *s, double *f, int where) {
     if (rc) return rc;
     if (!f) return fail(MDG_ERR_INVALID, "output pointer is null");
     if (!s->forces_valid) return fail(MDG_ERR_STATE, "no force evaluation since the last change");
+    if ((rc = enqueue_status(s))) return rc;
     CK(launch_forces_out(s), "forces out");
     CK(cudaMemcpyAsync(f, s->fout, sizeof(double) * 3 * s->n,
                        where == MDG_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                        s->stream),
        "copy forces");
-    CK(cudaStreamSynchronize(s->stream), "synchronize");
-    return read_status(s);
+    return finish_status(s);
 }
 
 MDG_API int mdg_get_energies_batch(mdg_system *s, double *energies, double *kinetic) {
     int rc = check_sys(s);
     if (rc) return rc;
-    std::vector<long long> e((size_t)kEnergySlots * s->n_sys);
-    CK(cudaMemcpyAsync(e.data(), s->energy, sizeof(long long) * e.size(), cudaMemcpyDeviceToHost,
-                       s->stream),
+    if ((rc = enqueue_status(s))) return rc;
+    const long long *e = s->host_stage;
+    CK(cudaMemcpyAsync(s->host_stage, s->energy, sizeof(long long) * stage_words(s),
+                       cudaMemcpyDeviceToHost, s->stream),
        "copy");
-    CK(cudaStreamSynchronize(s->stream), "synchronize");
-    rc = read_status(s);
+    rc = finish_status(s);
     if (rc) return rc;
     const bool recip = (s->forces_mask & MDG_MASK(MDG_TERM_COUL_RECIP)) && s->pme.on;
     for (int q = 0; q < s->n_sys; ++q) {
-        const long long *eq = e.data() + (size_t)kEnergySlots * q;
+        const long long *eq = e + (size_t)kEnergySlots * q;
         if (energies) {
             double *out = energies + (size_t)MDG_NUM_TERMS * q;
             for (int t = 0; t < MDG_NUM_TERMS; ++t) out[t] = (double)eq[t] * kFixInv;
@@ -1130,9 +1188,10 @@ MDG_API int mdg_kinetic_energy(mdg_system *s, double *kinetic) {
                          sizeof(long long), s->n_sys, s->stream),
        "memset");
     CK(launch_kinetic(s), "kinetic");
-    std::vector<long long> e((size_t)kEnergySlots * s->n_sys);
-    CK(cudaMemcpyAsync(e.data(), s->energy, sizeof(long long) * e.size(), cudaMemcpyDeviceToHost,
-                       s->stream),
+    if ((rc = stage_ready(s))) return rc;
+    const long long *e = s->host_stage;
+    CK(cudaMemcpyAsync(s->host_stage, s->energy, sizeof(long long) * stage_words(s),
+                       cudaMemcpyDeviceToHost, s->stream),
        "copy");
     CK(cudaStreamSynchronize(s->stream), "synchronize");
     double a = 0.0;
@@ -1399,9 +1458,7 @@ MDG_API int mdg_step_host(mdg_system *s, const double *x_in, const double *v_in,
         // pinned staging for the energy words, the status word and the
         // positions-comparison flag; each buffer is allocated once, so a
         // failed call leaves nothing half set up for the next one
-        if (!s->host_stage)
-            CK(cudaMallocHost((void **)&s->host_stage, sizeof(long long) * (ne + 2)),
-               "pinned staging");
+        if ((rc = stage_ready(s))) return rc;
         int rc2 = s->xin ? 0 : dalloc(&s->xin, 3 * (size_t)s->n);
         if (!rc2 && !s->same_flag) rc2 = dalloc(&s->same_flag, 1);
         if (rc2) return fail(rc2, "step_host staging");
@@ -1532,6 +1589,9 @@ MDG_API int mdg_set_mts(mdg_system *s, int k) {
     int rc = check_sys(s);
     if (rc) return rc;
     if (k < 1 || k > 16) return fail(MDG_ERR_INVALID, "outer step %d not in 1..16", k);
+    // the scheme in use: the forces and the captured steps stay (a program that
+    // integrates in short calls sets it before each)
+    if (s->mts_k == k && !ls_active(s)) return MDG_OK;
     s->mts_k = k;
     if (s->ls) s->ls->enabled = 0;
     s->forces_valid = 0;
@@ -1762,12 +1822,16 @@ MDG_API int mdg_integrator_config(mdg_system *s, int kind, double dt, double tem
     if (!(dt > 0)) return fail(MDG_ERR_INVALID, "time step must be positive");
     if (kind == MDG_INTEGRATOR_LANGEVIN && (!(temperature >= 0) || !(friction >= 0)))
         return fail(MDG_ERR_INVALID, "temperature and friction must be >= 0");
+    const double gamma = kind == MDG_INTEGRATOR_LANGEVIN ? friction : 0.0;
+    if (s->integ_kind == kind && s->dt == dt && s->temperature == temperature &&
+        s->friction == gamma && s->seed == seed)
+        return MDG_OK;  // the integrator in use: the captured steps stay
     s->integ_kind = kind;
     s->dt = dt;
     s->temperature = temperature;
-    s->friction = kind == MDG_INTEGRATOR_LANGEVIN ? friction : 0.0;
+    s->friction = gamma;
     s->seed = seed;
-    drop_graph(s);
+    drop_step_graphs(s);
     return MDG_OK;
 }
 
@@ -1797,13 +1861,11 @@ MDG_API int mdg_integrate(mdg_system *s, int n_steps, unsigned mask, int want_en
     rc = ready_for_forces(s, mask);
     if (rc) return rc;
     if (!s->have_masses) return fail(MDG_ERR_STATE, "masses have not been set");
-    if (s->graph.exec && s->graph.mask != mask) drop_graph(s);
+    if (s->graph.exec && s->graph.mask != mask) drop_step_graphs(s);
     for (auto &plane : s->graph_step)
         for (auto &row : plane)
             for (Graph &g : row)
-                if (g.exec && g.mask != mask) drop_graph(s);
-    for (Graph &g : s->graph_eval)
-        if (g.exec && g.mask != mask) drop_graph(s);
+                if (g.exec && g.mask != mask) drop_step_graphs(s);
     // the force buffer the first pre-force update uses: multiple time steps
     // want the weight of the evaluation that ended the previous step
     const float want_w = ls_active(s) ? -1.0f
@@ -1820,21 +1882,9 @@ MDG_API int mdg_integrate(mdg_system *s, int n_steps, unsigned mask, int want_en
             s->recip_weight = 1.0f;
             if (rc) return rc;
             s->forces_weight = want_w;
-        } else if (s->graph_mode == MDG_GRAPH_STEP && n_steps > 0) {
-            const int resort = s->need_reorder ? 1 : 0;
-            Graph &g = s->graph_eval[resort];
-            if (!g.exec) {
-                rc = capture_eval(s, g, resort, mask);
-                if (rc) return rc;
-            }
-            CK(cudaGraphLaunch(g.exec, s->stream), "graph launch");
-            s->launches += g.steps;
-            if (resort) {
-                s->need_reorder = 0;
-                s->steps_since_reorder = 0;
-            }
         } else {
-            rc = evaluate(s, mask, 1);
+            const bool step = s->graph_mode == MDG_GRAPH_STEP && n_steps > 0;
+            rc = run_evaluation(s, mask, step ? 0 : 1, step);
             if (rc) return rc;
         }
         s->forces_valid = 1;
@@ -1845,22 +1895,12 @@ MDG_API int mdg_integrate(mdg_system *s, int n_steps, unsigned mask, int want_en
     while (remaining > 0) {
         const bool chunk_start = s->need_reorder || s->steps_since_reorder >= R;
         const int usable = remaining - (want_energy ? 1 : 0);
-        if (s->graph_mode == MDG_GRAPH_STEP || s->mts_k > 1) {
-            const int e = (want_energy && remaining == 1) ? 1 : 0;
-            const int outer = mts_weight(s, s->step) != 0.f ? 1 : 0;
-            Graph &g = s->graph_step[chunk_start ? 1 : 0][e][outer];
-            if (!g.exec) {
-                rc = capture_steps(s, g, 1, chunk_start, mask, e);
-                if (rc) return rc;
-            }
-            CK(cudaGraphLaunch(g.exec, s->stream), "graph launch");
-            s->launches += g.steps;
-            s->need_reorder = 0;
-            s->steps_since_reorder = chunk_start ? 1 : s->steps_since_reorder + 1;
-            s->forces_weight = ls_active(s) ? -1.0f : mts_weight(s, s->step);
-            s->step += 1;
-            remaining -= 1;
-        } else if (chunk_start && usable >= R && R >= 2) {
+        // a whole chunk: one graph of R steps, captured when chunks keep coming
+        // (it holds R times a step's 20 nodes), else R single steps
+        const bool whole = s->graph_mode == MDG_GRAPH_CHUNK && s->mts_k == 1 && chunk_start &&
+                           usable >= R && R >= 2;
+        if (whole) s->chunk_uses += 1;
+        if (whole && (s->graph.exec || s->chunk_uses > 2 || usable >= 10 * R)) {
             if (!s->graph.exec) {
                 rc = capture_steps(s, s->graph, R, 1, mask);
                 if (rc) return rc;
@@ -1871,12 +1911,34 @@ MDG_API int mdg_integrate(mdg_system *s, int n_steps, unsigned mask, int want_en
             s->steps_since_reorder = R;
             s->step += R;
             remaining -= R;
-        } else {
-            const int e = (want_energy && remaining == 1) ? 1 : 0;
+            continue;
+        }
+        // a single step: its kind's graph, captured at once in step mode and
+        // with multiple time steps; otherwise when it comes up again (a capture
+        // costs about what four eager steps do)
+        const int e = (want_energy && remaining == 1) ? 1 : 0;
+        const int outer = mts_weight(s, s->step) != 0.f ? 1 : 0;
+        Graph &g = s->graph_step[chunk_start ? 1 : 0][e][outer];
+        const bool plain = !chunk_start && !e;
+        if (!g.exec && s->graph_mode == MDG_GRAPH_CHUNK && s->mts_k == 1 && g.uses < 2 &&
+            !(plain && remaining >= 6)) {
+            g.uses += 1;
             rc = md_step(s, mask, e);
             if (rc) return rc;
             remaining -= 1;
+            continue;
         }
+        if (!g.exec) {
+            rc = capture_steps(s, g, 1, chunk_start, mask, e);
+            if (rc) return rc;
+        }
+        CK(cudaGraphLaunch(g.exec, s->stream), "graph launch");
+        s->launches += g.steps;
+        s->need_reorder = 0;
+        s->steps_since_reorder = chunk_start ? 1 : s->steps_since_reorder + 1;
+        s->forces_weight = ls_active(s) ? -1.0f : mts_weight(s, s->step);
+        s->step += 1;
+        remaining -= 1;
     }
     if (want_energy && n_steps == 0) {
         rc = evaluate(s, mask, 1);

@@ -349,6 +349,7 @@ struct Graph {
     cudaGraphExec_t exec = nullptr;
     int steps = 0;
     unsigned mask = 0;
+    int uses = 0;  // runs without a graph since the last drop
 };
 
 // ---- learned slow force (multiple time steps) ------------------------------
@@ -507,7 +508,7 @@ struct mdg_system {
     unsigned long long *stats = nullptr;  // 4 counters
     unsigned long long *step_dev = nullptr;
     double *fout = nullptr;            // (n,3) FP64 staging for get_forces
-    long long *host_stage = nullptr;   // pinned host staging of mdg_step_host
+    long long *host_stage = nullptr;   // pinned host staging: energy words, status, a flag
     double *xin = nullptr;             // mdg_step_host: incoming positions (3n)
     double *vsave = nullptr;           // and the velocities before a speculative step
     int *same_flag = nullptr;          // and their comparison with the state
@@ -580,7 +581,8 @@ struct mdg_system {
     long long launches = 0;
     mdg::Graph graph;                  // chunk of reorder_interval steps
     mdg::Graph graph_step[2][2][2];    // one step: [re-sort first][with energies][MTS outer boundary]
-    mdg::Graph graph_eval[2];          // the evaluation before a first step: [re-sort first]
+    mdg::Graph graph_eval[2][2];       // one evaluation: [with energies][re-sort first]
+    int chunk_uses = 0;                // whole chunks run since the last drop
     int graph_mode = 0;
 
     // pair dump
