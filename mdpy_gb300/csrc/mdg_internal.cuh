@@ -231,8 +231,23 @@ struct PmeGroup {
     int count;
     long long grid_off, cgrid_off;
     long long nr_stride, nc_stride;  // elements between members' grids (padded)
+    bool own = false;                // transformed by mdg_fft.cu
     cufftHandle plan_f = 0, plan_b = 0;
     int *sys_ids = nullptr;  // device: the group's system ids, in grid order
+};
+
+// the systems whose transforms run in mdg_fft.cu
+struct FftBlock {             // what one block does: plane or column tile `index` of a system
+    int sys, index, K[3];
+    int tw[3], plan[3];       // twiddle factors and passes of the three lengths
+    long long grid_off, cgrid_off;
+};
+struct FftPlan {
+    int n_planes = 0, n_tiles = 0;
+    size_t plane_smem = 0, column_smem = 0;
+    FftBlock *planes = nullptr, *tiles = nullptr;  // device
+    float2 *tw = nullptr;
+    int4 *plan = nullptr;
 };
 
 struct Pme {
@@ -244,7 +259,8 @@ struct Pme {
     float *grid_r = nullptr;      // real grids (FFT input, then potential)
     float2 *grid_c = nullptr;     // half-spectrum complex grids
     float *influence = nullptr;   // influence functions, complex-grid layout
-    std::vector<PmeGroup> groups;
+    std::vector<PmeGroup> groups;  // own: transformed by `fft`, else by the group's plans
+    FftPlan fft;
 };
 
 // One warp packs cluster `warp`; lane slot k holds atom position c (FP64)
@@ -614,6 +630,10 @@ int prepare_sort_grid(mdg_system *s);   // host: column grid + cluster-order buf
 int pme_setup(mdg_system *s, const int *grids);  // host: grids, plans, influence functions
 int upload_sys_table(mdg_system *s);
 void pme_free(mdg_system *s);
+bool fft_supported(const int *K);       // mdg_fft.cu takes this grid
+void fft_free(FftPlan &f);
+int fft_setup(FftPlan &f, const std::vector<SysDev> &sys, const std::vector<int> &ids);
+cudaError_t fft_convolve(mdg_system *s, const FftPlan &f, int energy, int back);
 cudaError_t noalloc_scratch(int device, long long **out);  // static scratch of the no-alloc path
 cudaError_t launch_kinetic_scratch(mdg_system *s, long long *acc);
 // learned slow force (mdg_learned.cu)

@@ -13,6 +13,8 @@
 //              fixed-point adds into a shared-memory tile of the block's grid
 //              patch, then one global red.add per tile point (order
 //              independent);
+//   mdg_fft.cu the transforms of small grids, influence function included, in
+//              three launches for a whole batch; larger grids:
 //   k_grid_convert  int64 grid -> float grid, and re-zeroes the int64 grid;
 //   cuFFT R2C  (the only library call of the path);
 //   k_convolve multiply by the influence function; optional energy sum;
@@ -160,7 +162,7 @@ __device__ __forceinline__ size_t patch_point(const Patch &sp, int t, int ey, in
     return ((size_t)gx * K1 + gy) * K2 + gz;
 }
 
-// Charge spreading.  Atoms arrive in cluster order, so a block's atoms sit in
+// Charge spreading through tiles.  Atoms arrive in cluster order, so a block's atoms sit in
 // a compact patch of the grid: the block accumulates its p^3 contributions per
 // atom into an int64 tile in shared memory (shared atomics) and then adds each
 // nonzero tile point to the system's grid with one global atomic -- about 30
@@ -415,6 +417,7 @@ void pme_free(mdg_system *s) {
         if (g.sys_ids) cudaFree(g.sys_ids);
     }
     p.groups.clear();
+    fft_free(p.fft);
     cudaFree(p.grid_i);
     cudaFree(p.grid_r);
     cudaFree(p.grid_c);
@@ -506,11 +509,14 @@ int pme_setup(mdg_system *s, const int *grids) {
     const double pi = 3.14159265358979323846;
     const double b2 = p.beta * p.beta;
     std::vector<float> G(coff);
+    std::vector<int> own;  // systems whose transforms run in mdg_fft.cu
     for (size_t g = 0; g < members.size(); ++g) {
         PmeGroup &grp = p.groups[g];
         const int K0 = grp.K[0], K1 = grp.K[1], K2 = grp.K[2], Kh = K2 / 2 + 1;
         int n[3] = {K0, K1, K2}, nh[3] = {K0, K1, Kh};
-        if (cufftPlanMany(&grp.plan_f, 3, n, n, 1, (int)grp.nr_stride, nh, 1, (int)grp.nc_stride,
+        grp.own = fft_supported(grp.K);
+        if (grp.own) own.insert(own.end(), members[g].begin(), members[g].end());
+        else if (cufftPlanMany(&grp.plan_f, 3, n, n, 1, (int)grp.nr_stride, nh, 1, (int)grp.nc_stride,
                           CUFFT_R2C, grp.count) != CUFFT_SUCCESS ||
             cufftPlanMany(&grp.plan_b, 3, n, nh, 1, (int)grp.nc_stride, n, 1, (int)grp.nr_stride,
                           CUFFT_C2R, grp.count) != CUFFT_SUCCESS)
@@ -546,7 +552,8 @@ int pme_setup(mdg_system *s, const int *grids) {
     if (cudaMemcpy(p.influence, G.data(), coff * sizeof(float), cudaMemcpyHostToDevice) !=
         cudaSuccess)
         return MDG_ERR_CUDA;
-    return upload_sys_table(s);
+    const int rc = fft_setup(p.fft, s->sys_h, own);
+    return rc ? rc : upload_sys_table(s);
 }
 
 cudaError_t launch_pme(mdg_system *s, int energy, int *cufft_status) {
@@ -577,10 +584,20 @@ cudaError_t launch_pme(mdg_system *s, int energy, int *cufft_status) {
         case 6: k_spread<6><<<nb, ab, spread_smem, st>>>(a); break;
         default: return cudaErrorInvalidValue;
     }
-    k_grid_convert<<<(unsigned)((p.grid_total + tb - 1) / tb), tb, 0, st>>>(p.grid_i, p.grid_r,
-                                                                            p.grid_total);
-    s->launches += 2;
+    s->launches += 1;
+    // weight 0 (an impulse inner step that only reports the energy): the
+    // potential grid is never gathered, so the way back is skipped
+    cudaError_t fe = fft_convolve(s, p.fft, energy, a.weight != 0.f);
+    if (fe != cudaSuccess) return fe;
     for (PmeGroup &g : p.groups) {
+        if (g.own) continue;
+        const long long n = g.nr_stride * g.count;
+        k_grid_convert<<<(unsigned)((n + tb - 1) / tb), tb, 0, st>>>(p.grid_i + g.grid_off,
+                                                                     p.grid_r + g.grid_off, n);
+        s->launches += 1;
+    }
+    for (PmeGroup &g : p.groups) {
+        if (g.own) continue;
         cufftResult r = cufftSetStream(g.plan_f, st);
         if (r == CUFFT_SUCCESS)
             r = cufftExecR2C(g.plan_f, p.grid_r + g.grid_off, (cufftComplex *)(p.grid_c + g.cgrid_off));
@@ -590,6 +607,7 @@ cudaError_t launch_pme(mdg_system *s, int energy, int *cufft_status) {
         }
     }
     for (PmeGroup &g : p.groups) {
+        if (g.own) continue;
         const int Kh = g.K[2] / 2 + 1;
         const long long nc = g.nc_stride;  // padding elements carry G = 0
         const long long totc = nc * g.count;
@@ -603,10 +621,9 @@ cudaError_t launch_pme(mdg_system *s, int energy, int *cufft_status) {
                                                   g.sys_ids, s->energy);
         s->launches += 1;
     }
-    // weight 0 (an impulse inner step that only reports the energy): the
-    // potential grid is never gathered, so the backward transform is skipped
     for (PmeGroup &g : p.groups) {
         if (a.weight == 0.f) break;
+        if (g.own) continue;
         cufftResult r = cufftSetStream(g.plan_b, st);
         if (r == CUFFT_SUCCESS)
             r = cufftExecC2R(g.plan_b, (cufftComplex *)(p.grid_c + g.cgrid_off), p.grid_r + g.grid_off);
