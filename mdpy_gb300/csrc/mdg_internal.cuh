@@ -54,6 +54,22 @@ __device__ __forceinline__ void raise_status(int *status, int code) {
 }
 
 __device__ __forceinline__ long long to_fix(float v) { return __float2ll_rn(v * kFixScaleF); }
+// the same value from FP32 adds, for |v| < 63 (larger values, infinities and NaN
+// take the conversion).  A 64-bit conversion runs on the FP64 pipe, 16 cycles a
+// warp and SM; these ten instructions pay where conversions are most of the work
+// (charge spreading), not in the pair kernel.  hi = v 2^16 rounded to an integer
+// (the sum with 1.5 2^23 keeps it in the low mantissa bits), what is left of
+// v 2^16 is exact, and its product with 2^16 rounds once; hi 2^16 is even, so
+// ties break as in the direct conversion.
+__device__ __forceinline__ long long to_fix_alu(float v) {
+    if (!(fabsf(v) < 63.0f)) return to_fix(v);
+    const float m = 12582912.0f;  // 1.5 2^23
+    const float t1 = __fmaf_rn(v, 65536.0f, m);
+    const float r = __fmaf_rn(v, 65536.0f, -__fsub_rn(t1, m));
+    const float t2 = __fmaf_rn(r, 65536.0f, m);
+    const int hi = __float_as_int(t1) - 0x4B400000, lo = __float_as_int(t2) - 0x4B400000;
+    return (long long)hi * 65536ll + (long long)lo;
+}
 __device__ __forceinline__ long long to_fix_d(double v) { return __double2ll_rn(v * kFixScale); }
 
 // fire-and-forget 64-bit add into a fixed-point accumulator (two's complement)
