@@ -78,11 +78,12 @@ void drop_one(Graph &g) {
 }
 
 void drop_step_graphs(mdg_system *s) {
-    drop_one(s->graph);
+    for (Graph &g : s->graph) drop_one(g);
     s->chunk_uses = 0;
-    for (auto &plane : s->graph_step)
-        for (auto &row : plane)
-            for (Graph &g : row) drop_one(g);
+    for (auto &pending : s->graph_step)
+        for (auto &plane : pending)
+            for (auto &row : plane)
+                for (Graph &g : row) drop_one(g);
 }
 
 void drop_graph(mdg_system *s) {
@@ -232,6 +233,8 @@ int evaluate(mdg_system *s, unsigned mask, int energy) {
     if (!rc && e == cudaSuccess && lsp != kLsOff) e = ls_side(s, lsp);
     cudaError_t ej = cudaEventRecord(s->ev_join, s->side_stream);
     s->stream = s->bond_stream;
+    if (!rc && e == cudaSuccess && s->count_step) e = launch_count_step(s);
+    s->count_step = 0;
     if (!rc && e == cudaSuccess) e = launch_special(s, mask, energy, 0);
     if (!rc && e == cudaSuccess) e = launch_bonded(s, mask, energy);
     cudaError_t ej2 = cudaEventRecord(s->ev_join2, s->bond_stream);
@@ -272,11 +275,15 @@ float mts_weight(const mdg_system *s, uint64_t step) {
     return ((step + 1) % (uint64_t)s->mts_k == 0) ? (float)s->mts_k : 0.0f;
 }
 
-int md_step(mdg_system *s, unsigned mask, int energy) {
-    // (the pre-force update stays its own coalesced pass over atom order: a
-    // version fused into the cluster-order packing measured 1 % slower)
-    CK(launch_integrate_pre(s), "integrate pre");
+// One step.  The first kernel is the pre-force update, behind the kick that the
+// step before left pending; the last step of a run kicks at once.
+int md_step(mdg_system *s, unsigned mask, StepEnd end) {
+    const int energy = end == kLastEnergy ? 1 : 0;
+    const bool pending = s->post_pending != 0;
     if (s->steps_since_reorder >= s->reorder_interval) s->need_reorder = 1;
+    CK(launch_move(s, pending), "integrate");
+    s->count_step = pending ? 1 : 0;
+    s->post_pending = 0;
     int rc;
     if (ls_active(s)) {
         rc = ls_evaluate(s, mask, energy, mts_weight(s, s->step) != 0.f ? kLsOuter : kLsInner);
@@ -287,31 +294,35 @@ int md_step(mdg_system *s, unsigned mask, int energy) {
         s->recip_weight = 1.0f;
     }
     if (rc) return rc;
-    CK(launch_integrate_post(s, energy), "integrate post");
+    if (end != kMid) CK(launch_integrate_post(s, energy), "integrate post");
+    else s->post_pending = 1;
     s->steps_since_reorder += 1;
     s->step += 1;
     return MDG_OK;
 }
 
-// Capture `nsteps` MD steps (the first re-sorting the atoms when `resort`)
-// into g; host-side counters are restored, the launch count per replay is
-// kept in g.steps.
-int capture_steps(mdg_system *s, Graph &g, int nsteps, int resort, unsigned mask,
-                  int energy_last = 0) {
+// Capture `nsteps` MD steps (the first re-sorting the atoms when `resort`, and
+// kicking first when `pending`; the last as `end` says) into g; host-side
+// counters are restored, the launch count per replay is kept in g.steps.
+int capture_steps(mdg_system *s, Graph &g, int nsteps, int resort, unsigned mask, int pending,
+                  StepEnd end) {
     const long long saved = s->launches;
     const int saved_since = s->steps_since_reorder, saved_need = s->need_reorder;
     const uint64_t saved_step = s->step;
+    const int saved_pending = s->post_pending;
+    s->post_pending = pending;
     s->need_reorder = resort ? 1 : 0;
     if (!resort) s->steps_since_reorder = 0;
     CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal), "capture");
     int crc = MDG_OK;
     for (int k = 0; k < nsteps && !crc; ++k)
-        crc = md_step(s, mask, (energy_last && k == nsteps - 1) ? 1 : 0);
+        crc = md_step(s, mask, k == nsteps - 1 ? end : kMid);
     cudaGraph_t graph = nullptr;
     cudaError_t ce = cudaStreamEndCapture(s->stream, &graph);
     s->steps_since_reorder = saved_since;
     s->need_reorder = saved_need;
     s->step = saved_step;
+    s->post_pending = saved_pending;
     const long long per = s->launches - saved;
     s->launches = saved;
     if (crc) {
@@ -490,6 +501,7 @@ MDG_API int mdg_system_create_batch(int device, int n_systems, const int *n_atom
     }
     AL(s->mass, n);
     AL(s->inv_mass, n);
+    AL(s->sqrt_mass, n);
     AL(s->charge, n);
     AL(s->lj, n);
     AL(s->inv_perm, n);
@@ -523,6 +535,7 @@ MDG_API int mdg_system_create_batch(int device, int n_systems, const int *n_atom
     std::vector<double> ones(n, 1.0);
     cudaMemcpy(s->mass, ones.data(), sizeof(double) * n, cudaMemcpyHostToDevice);
     cudaMemcpy(s->inv_mass, ones.data(), sizeof(double) * n, cudaMemcpyHostToDevice);
+    cudaMemcpy(s->sqrt_mass, ones.data(), sizeof(double) * n, cudaMemcpyHostToDevice);
     s->pw = 0;
     rc = prepare_sort_grid(s);
     if (rc) {
@@ -552,6 +565,7 @@ MDG_API int mdg_system_destroy(mdg_system *s) {
     pme_free(s);
     dfree(s->mass);
     dfree(s->inv_mass);
+    dfree(s->sqrt_mass);
     dfree(s->charge);
     dfree(s->lj);
     dfree(s->partners);
@@ -684,13 +698,15 @@ MDG_API int mdg_system_set_boxes(mdg_system *s, const double *boxes) {
 MDG_API int mdg_set_masses(mdg_system *s, const double *m) {
     int rc = check_sys(s);
     if (rc) return rc;
-    std::vector<double> mm(m, m + s->n), inv(s->n);
+    std::vector<double> mm(m, m + s->n), inv(s->n), root(s->n);
     for (int i = 0; i < s->n; ++i) {
         if (!(mm[i] > 0)) return fail(MDG_ERR_INVALID, "mass of atom %d is %g", i, mm[i]);
         inv[i] = 1.0 / mm[i];
+        root[i] = std::sqrt(mm[i]);
     }
     CK(cudaMemcpy(s->mass, mm.data(), sizeof(double) * s->n, cudaMemcpyHostToDevice), "copy");
     CK(cudaMemcpy(s->inv_mass, inv.data(), sizeof(double) * s->n, cudaMemcpyHostToDevice), "copy");
+    CK(cudaMemcpy(s->sqrt_mass, root.data(), sizeof(double) * s->n, cudaMemcpyHostToDevice), "copy");
     s->have_masses = 1;
     return MDG_OK;
 }
@@ -1341,7 +1357,7 @@ MDG_API int mdg_autotune(mdg_system *s, unsigned mask, int reps, double *best_ms
             cudaMemcpyAsync(s->v, vs, sizeof(double) * 3 * s->n, cudaMemcpyDeviceToDevice,
                             s->stream);
             r = evaluate(s, mask, 0);  // forces of the restored positions
-            if (!r) r = capture_steps(s, g, 1, 0, mask);
+            if (!r) r = capture_steps(s, g, 1, 0, mask, 0, kLast);
         }
         float total = 0.f;
         for (int w = 0; w < 2 + n && !r && ce == cudaSuccess; ++w) {
@@ -1861,11 +1877,19 @@ MDG_API int mdg_integrate(mdg_system *s, int n_steps, unsigned mask, int want_en
     rc = ready_for_forces(s, mask);
     if (rc) return rc;
     if (!s->have_masses) return fail(MDG_ERR_STATE, "masses have not been set");
-    if (s->graph.exec && s->graph.mask != mask) drop_step_graphs(s);
-    for (auto &plane : s->graph_step)
-        for (auto &row : plane)
-            for (Graph &g : row)
-                if (g.exec && g.mask != mask) drop_step_graphs(s);
+    for (Graph &g : s->graph)
+        if (g.exec && g.mask != mask) drop_step_graphs(s);
+    for (auto &pending : s->graph_step)
+        for (auto &plane : pending)
+            for (auto &row : plane)
+                for (Graph &g : row)
+                    if (g.exec && g.mask != mask) drop_step_graphs(s);
+    s->count_step = 0;
+    // a run that an error cut short: its last step's kick
+    if (s->post_pending) {
+        s->post_pending = 0;
+        CK(launch_integrate_post(s, 0), "integrate post");
+    }
     // the force buffer the first pre-force update uses: multiple time steps
     // want the weight of the evaluation that ended the previous step
     const float want_w = ls_active(s) ? -1.0f
@@ -1900,13 +1924,15 @@ MDG_API int mdg_integrate(mdg_system *s, int n_steps, unsigned mask, int want_en
         const bool whole = s->graph_mode == MDG_GRAPH_CHUNK && s->mts_k == 1 && chunk_start &&
                            usable >= R && R >= 2;
         if (whole) s->chunk_uses += 1;
-        if (whole && (s->graph.exec || s->chunk_uses > 2 || usable >= 10 * R)) {
-            if (!s->graph.exec) {
-                rc = capture_steps(s, s->graph, R, 1, mask);
+        Graph &gc = s->graph[s->post_pending];
+        if (whole && (gc.exec || s->chunk_uses > 2 || usable >= 10 * R)) {
+            if (!gc.exec) {
+                rc = capture_steps(s, gc, R, 1, mask, s->post_pending, kMid);
                 if (rc) return rc;
             }
-            CK(cudaGraphLaunch(s->graph.exec, s->stream), "graph launch");
-            s->launches += s->graph.steps;
+            CK(cudaGraphLaunch(gc.exec, s->stream), "graph launch");
+            s->launches += gc.steps;
+            s->post_pending = 1;
             s->need_reorder = 0;
             s->steps_since_reorder = R;
             s->step += R;
@@ -1916,29 +1942,34 @@ MDG_API int mdg_integrate(mdg_system *s, int n_steps, unsigned mask, int want_en
         // a single step: its kind's graph, captured at once in step mode and
         // with multiple time steps; otherwise when it comes up again (a capture
         // costs about what four eager steps do)
-        const int e = (want_energy && remaining == 1) ? 1 : 0;
+        const StepEnd end = remaining > 1 ? kMid : want_energy ? kLastEnergy : kLast;
         const int outer = mts_weight(s, s->step) != 0.f ? 1 : 0;
-        Graph &g = s->graph_step[chunk_start ? 1 : 0][e][outer];
-        const bool plain = !chunk_start && !e;
+        Graph &g = s->graph_step[s->post_pending][chunk_start ? 1 : 0][end][outer];
+        const bool plain = !chunk_start && end == kMid && s->post_pending;
         if (!g.exec && s->graph_mode == MDG_GRAPH_CHUNK && s->mts_k == 1 && g.uses < 2 &&
             !(plain && remaining >= 6)) {
             g.uses += 1;
-            rc = md_step(s, mask, e);
+            rc = md_step(s, mask, end);
             if (rc) return rc;
             remaining -= 1;
             continue;
         }
         if (!g.exec) {
-            rc = capture_steps(s, g, 1, chunk_start, mask, e);
+            rc = capture_steps(s, g, 1, chunk_start, mask, s->post_pending, end);
             if (rc) return rc;
         }
         CK(cudaGraphLaunch(g.exec, s->stream), "graph launch");
         s->launches += g.steps;
+        s->post_pending = end == kMid ? 1 : 0;
         s->need_reorder = 0;
         s->steps_since_reorder = chunk_start ? 1 : s->steps_since_reorder + 1;
         s->forces_weight = ls_active(s) ? -1.0f : mts_weight(s, s->step);
         s->step += 1;
         remaining -= 1;
+    }
+    if (s->post_pending) {  // the run ended with a chunk
+        s->post_pending = 0;
+        CK(launch_integrate_post(s, 0), "integrate post");
     }
     if (want_energy && n_steps == 0) {
         rc = evaluate(s, mask, 1);
@@ -2060,7 +2091,7 @@ MDG_API int mdg_launch_stage(mdg_system *s, int stage, unsigned mask) {
         case MDG_STAGE_REORDER: CK(launch_reorder(s), "reorder"); break;
         case MDG_STAGE_INTEGRATE:
             if (s->integ_kind < 0) return fail(MDG_ERR_STATE, "integrator not configured");
-            CK(launch_integrate_pre(s), "pre");
+            CK(launch_move(s, false), "pre");
             CK(launch_integrate_post(s, 0), "post");
             break;
         default: return fail(MDG_ERR_INVALID, "unknown stage %d", stage);

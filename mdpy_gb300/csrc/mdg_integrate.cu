@@ -5,8 +5,9 @@
 // and LangevinIntegrator.integrate (mdpy/integrator/langevin_integrator.py:37-71)
 // plus Ensemble._update_kinetic_energy (mdpy/ensemble.py:63-71).
 //
-// Both integrators are written as one "pre-force" and one "post-force" kernel
-// around a single force evaluation per step:
+// Both integrators are written as one "pre-force" and one "post-force" update
+// around a single force evaluation per step; inside a run a step's post-force
+// update and the next step's pre-force update are one kernel (k_move):
 //   pre :  x += b dt v + b dt^2/(2m) F_n + b dt/(2m) beta
 //          v  = a v + a dt/(2m) F_n + b/m beta
 //   post:  v += dt/(2m) F_{n+1}
@@ -53,10 +54,11 @@ struct InArgs {
     double *__restrict__ v;
     const double *__restrict__ mass;
     const double *__restrict__ inv_mass;
+    const double *__restrict__ sqrt_mass;
     const int *__restrict__ inv_perm;
-    const unsigned long long *__restrict__ f;
+    const unsigned long long *f;
     int n, n_pad;
-    double dt, ca, cb, noise;  // noise = sqrt(2 gamma kT dt)
+    double dt, half_dt, ca, cb, noise;  // noise = sqrt(2 gamma kT dt)
     int langevin;
     unsigned long long seed;
     unsigned long long *step;
@@ -69,39 +71,57 @@ __device__ __forceinline__ double fget(const unsigned long long *f, int k) {
     return (double)(long long)f[k] * kFixInv;
 }
 
-// the pre-force update of atom i (cluster slot k) from the forces in slot k
-__device__ __forceinline__ void pre_kick(const InArgs &a, int i, int k) {
+// no FP64 compare: an exponent of all ones is an infinity or NaN
+__device__ __forceinline__ bool finite_bits(double v) {
+    return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000;
+}
+
+// The updates of atom i around the forces in its cluster slot k, one thread per
+// atom: with POST the kick that ends a step, then the pre-force update of the
+// next step.  Bound by the FP64 pipe (two lanes per clock and SM), so the forces
+// stay integers times 2^-32 (an exact factor of the coefficients), the root of
+// the mass is read, finiteness is read off the exponents, and the two updates
+// share their loads and conversions: 39 FP64-pipe operations an atom (85 before,
+// as two kernels).  The sums round as they did there.
+template <bool POST>
+__global__ void __launch_bounds__(256) k_move(InArgs a) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= a.n) return;
+    const int k = a.inv_perm[i];
     const double im = a.inv_mass[i];
-    const double F[3] = {fget(a.f, k), fget(a.f, a.n_pad + k), fget(a.f, 2 * a.n_pad + k)};
+    const double F[3] = {(double)(long long)a.f[k], (double)(long long)a.f[a.n_pad + k],
+                         (double)(long long)a.f[2 * a.n_pad + k]};
+    const double h = a.half_dt * im;    // dt / (2m)
+    const double hf = h * kFixInv;      // of a fixed-point force
     double bt[3] = {0.0, 0.0, 0.0};
     if (a.langevin) {
-        const float3 g = gauss3((unsigned)i, *a.step, a.seed);
-        const double sm = sqrt(a.mass[i]) * a.noise;
+        // with POST the step counter moves on later in this step (k_count_step)
+        const float3 g = gauss3((unsigned)i, *a.step + (POST ? 1ull : 0ull), a.seed);
+        const double sm = a.sqrt_mass[i] * a.noise;
         bt[0] = sm * g.x;
         bt[1] = sm * g.y;
         bt[2] = sm * g.z;
     }
-    const double h = 0.5 * a.dt * im;
     bool ok = true;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        const double v0 = a.v[3 * i + d];
-        // b dt v + b dt^2/(2m) F + b dt/(2m) beta   (h = dt/(2m))
-        const double xn = a.x[3 * i + d] + a.cb * (a.dt * (v0 + h * F[d]) + h * bt[d]);
-        const double vn = a.ca * v0 + a.ca * h * F[d] + a.cb * im * bt[d];
-        ok = ok && isfinite(xn) && isfinite(vn);
+        double v0 = a.v[3 * i + d];
+        if (POST) v0 = v0 + hf * F[d];
+        // b dt v + b dt^2/(2m) F + b dt/(2m) beta
+        double xn = a.dt * (v0 + hf * F[d]), vn = a.ca * v0 + a.ca * hf * F[d];
+        if (a.langevin) {
+            xn = a.dt * (v0 + hf * F[d]) + h * bt[d];
+            vn = a.ca * v0 + a.ca * hf * F[d] + a.cb * im * bt[d];
+        }
+        xn = a.x[3 * i + d] + a.cb * xn;
+        ok = ok && finite_bits(xn) && finite_bits(vn);
         a.x[3 * i + d] = xn;
         a.v[3 * i + d] = vn;
     }
     if (!ok) raise_status(a.status, MDG_ERR_PARTICLE_LOSS);
 }
 
-__global__ void __launch_bounds__(256) k_pre(InArgs a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
-    pre_kick(a, i, a.inv_perm[i]);
-}
-
+__global__ void k_count_step(unsigned long long *step) { *step += 1ull; }
 
 template <bool ENERGY>
 __global__ void __launch_bounds__(256) k_post(InArgs a) {
@@ -109,11 +129,11 @@ __global__ void __launch_bounds__(256) k_post(InArgs a) {
     double ke = 0.0;
     if (i < a.n) {
         const int k = a.inv_perm[i];
-        const double h = 0.5 * a.dt * a.inv_mass[i];
+        const double hf = a.half_dt * a.inv_mass[i] * kFixInv;
         double vv = 0.0;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            const double vn = a.v[3 * i + d] + h * fget(a.f, d * a.n_pad + k);
+            const double vn = a.v[3 * i + d] + hf * (double)(long long)a.f[d * a.n_pad + k];
             a.v[3 * i + d] = vn;
             vv += vn * vn;
         }
@@ -209,11 +229,13 @@ InArgs make_args(mdg_system *s) {
     a.v = s->v;
     a.mass = s->mass;
     a.inv_mass = s->inv_mass;
+    a.sqrt_mass = s->sqrt_mass;
     a.inv_perm = s->inv_perm;
     a.f = s->f;
     a.n = s->n;
     a.n_pad = s->n_pad;
     a.dt = s->dt;
+    a.half_dt = 0.5 * s->dt;
     const bool lg = s->integ_kind == MDG_INTEGRATOR_LANGEVIN && s->friction > 0;
     const double g = lg ? s->friction : 0.0;
     a.ca = (1.0 - 0.5 * g * s->dt) / (1.0 + 0.5 * g * s->dt);
@@ -232,19 +254,33 @@ InArgs make_args(mdg_system *s) {
 
 }  // namespace
 
-cudaError_t launch_integrate_pre(mdg_system *s) {
-    InArgs a = make_args(s);
-    k_pre<<<(s->n + 255) / 256, 256, 0, s->stream>>>(a);
+// Threads per block of the updates: their FP64 work runs at two lanes per clock
+// and SM, so few atoms are spread over many SMs.
+int move_threads(const mdg_system *s) { return s->n < 64 * 8 * s->n_sms ? 64 : 256; }
+
+// The pre-force update, with `post` behind the kick that ended the step before.
+// (With the packing of the new positions in the same kernel, in cluster order, a
+// step took as long at 2,700 atoms and 5 % longer at 20,000.)
+cudaError_t launch_move(mdg_system *s, bool post) {
+    const InArgs a = make_args(s);
+    const int tb = move_threads(s), nb = (s->n + tb - 1) / tb;
+    if (post) k_move<true><<<nb, tb, 0, s->stream>>>(a);
+    else k_move<false><<<nb, tb, 0, s->stream>>>(a);
+    s->launches += 1;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_count_step(mdg_system *s) {
+    k_count_step<<<1, 1, 0, s->stream>>>(s->step_dev);
     s->launches += 1;
     return cudaGetLastError();
 }
 
 cudaError_t launch_integrate_post(mdg_system *s, int energy) {
     InArgs a = make_args(s);
-    if (energy)
-        k_post<true><<<(s->n + 255) / 256, 256, 0, s->stream>>>(a);
-    else
-        k_post<false><<<(s->n + 255) / 256, 256, 0, s->stream>>>(a);
+    const int tb = move_threads(s), nb = (s->n + tb - 1) / tb;
+    if (energy) k_post<true><<<nb, tb, 0, s->stream>>>(a);
+    else k_post<false><<<nb, tb, 0, s->stream>>>(a);
     s->launches += 1;
     return cudaGetLastError();
 }

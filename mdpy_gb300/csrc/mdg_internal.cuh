@@ -377,6 +377,9 @@ __device__ __forceinline__ void pack_cluster(const PackArgs &a, int warp, int k,
     }
 }
 
+// where a step stands in its run: more follow, the last, the last with energies
+enum StepEnd { kMid = 0, kLast = 1, kLastEnergy = 2 };
+
 struct Graph {
     cudaGraphExec_t exec = nullptr;
     int steps = 0;
@@ -501,7 +504,7 @@ struct mdg_system {
                                        // of their columns since the last re-sort
 
     // static, atom order
-    double *mass = nullptr, *inv_mass = nullptr;
+    double *mass = nullptr, *inv_mass = nullptr, *sqrt_mass = nullptr;
     float *charge = nullptr;          // q * sqrt(k_e)
     float4 *lj = nullptr;             // sigma/2, sqrt(4 eps), sigma14/2, sqrt(4 eps14)
     int pw = 0;                       // partner width
@@ -611,8 +614,13 @@ struct mdg_system {
     int evaluated_once = 0;
     unsigned forces_mask = 0;
     long long launches = 0;
-    mdg::Graph graph;                  // chunk of reorder_interval steps
-    mdg::Graph graph_step[2][2][2];    // one step: [re-sort first][with energies][MTS outer boundary]
+    // Inside a run the kick that ends a step waits for the next step's first
+    // kernel (post_pending); a run ends with it done.
+    int post_pending = 0;
+    int count_step = 0;                // the evaluation under way moves the step counter on
+    mdg::Graph graph[2];               // chunk of reorder_interval steps: [kick pending]
+    // one step: [kick pending][re-sort first][kMid, kLast, kLastEnergy][MTS outer boundary]
+    mdg::Graph graph_step[2][2][3][2];
     mdg::Graph graph_eval[2][2];       // one evaluation: [with energies][re-sort first]
     int chunk_uses = 0;                // whole chunks run since the last drop
     int graph_mode = 0;
@@ -634,7 +642,8 @@ int nb_parts(const mdg_system *s);  // work items per cluster of the pair kernel
 cudaError_t launch_special(mdg_system *s, unsigned mask, int energy, int dump);
 cudaError_t launch_pme(mdg_system *s, int energy, int *cufft_status);
 cudaError_t launch_bonded(mdg_system *s, unsigned mask, int energy);
-cudaError_t launch_integrate_pre(mdg_system *s);
+cudaError_t launch_move(mdg_system *s, bool post);
+cudaError_t launch_count_step(mdg_system *s);
 cudaError_t launch_integrate_post(mdg_system *s, int energy);
 cudaError_t launch_kinetic(mdg_system *s);
 cudaError_t launch_forces_out(mdg_system *s);
