@@ -506,6 +506,7 @@ MDG_API int mdg_system_create_batch(int device, int n_systems, const int *n_atom
     AL(s->lj, n);
     AL(s->inv_perm, n);
     AL(s->atom_key, n);
+    AL(s->atom_order, n);
     AL(s->tmp_perm, n);
     AL(s->atom_sys, n);
     AL(s->x, 3 * (size_t)n);
@@ -580,7 +581,7 @@ MDG_API int mdg_system_destroy(mdg_system *s) {
     dfree(s->cell_rank);
     dfree(s->cell_count);
     dfree(s->cell_start);
-    dfree(s->cell_cursor);
+    dfree(s->atom_order);
     dfree(s->atom_key);
     dfree(s->tmp_perm);
     dfree(s->atom_sys);

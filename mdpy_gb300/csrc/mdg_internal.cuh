@@ -528,7 +528,7 @@ struct mdg_system {
     int n_cols = 0;
     int *col_ncl = nullptr, *col_cl_start = nullptr;
     int *cell_rank = nullptr, *cell_count = nullptr, *cell_start = nullptr,
-        *cell_cursor = nullptr, *atom_key = nullptr, *tmp_perm = nullptr, *scan_blocks = nullptr;
+        *atom_key = nullptr, *atom_order = nullptr, *tmp_perm = nullptr, *scan_blocks = nullptr;
     int n_scan_blocks = 0;
 
     // per step
