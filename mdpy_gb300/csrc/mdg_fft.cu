@@ -202,6 +202,7 @@ __global__ void __launch_bounds__(kPlaneThreads) k_fft_planes(FftArgs a) {
     const unsigned mg_h = magic_of(Kh);
     const size_t real0 = b.grid_off + (size_t)b.index * K1 * K2;
     float2 *const gc = a.gc + b.cgrid_off + (size_t)b.index * K1 * Kh;
+    wait_for_previous();  // (the tables above do not change)
     if constexpr (!INV) {
         // two z lines (y = 2 p and 2 p + 1) as one complex line
         long long *const gi = a.gi + real0;
@@ -292,12 +293,16 @@ __global__ void __launch_bounds__(128) k_fft_columns(FftArgs a) {
     float2 *const gc = a.gc + b.cgrid_off + c0;
     const float *const G = a.G + b.cgrid_off + c0;
     constexpr unsigned mg_c = (unsigned)(0x100000000ull / kCols);
-    // (the influence function's loads beside the spectrum's)
+#pragma unroll 4
+    for (int t = threadIdx.x; t < kCols * K0; t += blockDim.x) {
+        const int x = t / kCols, c = t % kCols;
+        sG[t] = c < nc ? G[(size_t)x * plane + c] : 0.f;
+    }
+    wait_for_previous();  // (tables and influence function do not change)
 #pragma unroll 4
     for (int t = threadIdx.x; t < kCols * K0; t += blockDim.x) {
         const int x = t / kCols, c = t % kCols;
         A[t] = c < nc ? gc[(size_t)x * plane + c] : make_float2(0.f, 0.f);
-        sG[t] = c < nc ? G[(size_t)x * plane + c] : 0.f;
     }
     __syncthreads();
     float2 *r = fft_lines<false, false>(A, B, tw, s_plan, K0, kCols, mg_c, 1, kCols);
@@ -434,18 +439,20 @@ cudaError_t fft_convolve(mdg_system *s, const FftPlan &f, int energy, int back) 
     a.energy = s->energy;
     cudaStream_t st = s->stream;
     a.blocks = f.planes;
-    k_fft_planes<false><<<f.n_planes, kPlaneThreads, f.plane_smem, st>>>(a);
+    cudaError_t e = launch_after(k_fft_planes<false>, f.n_planes, kPlaneThreads, f.plane_smem, st, a);
     FftArgs c = a;
     c.blocks = f.tiles;
-    if (!back) k_fft_columns<true, false><<<f.n_tiles, 128, f.column_smem, st>>>(c);
-    else if (energy) k_fft_columns<true, true><<<f.n_tiles, 128, f.column_smem, st>>>(c);
-    else k_fft_columns<false, true><<<f.n_tiles, 128, f.column_smem, st>>>(c);
+    if (e == cudaSuccess)
+        e = launch_after(!back    ? k_fft_columns<true, false>
+                         : energy ? k_fft_columns<true, true>
+                                  : k_fft_columns<false, true>,
+                         f.n_tiles, 128, f.column_smem, st, c);
     s->launches += 2;
-    if (back) {
-        k_fft_planes<true><<<f.n_planes, kPlaneThreads, f.plane_smem, st>>>(a);
+    if (back && e == cudaSuccess) {
+        e = launch_after(k_fft_planes<true>, f.n_planes, kPlaneThreads, f.plane_smem, st, a);
         s->launches += 1;
     }
-    return cudaGetLastError();
+    return e;
 }
 
 }  // namespace mdg

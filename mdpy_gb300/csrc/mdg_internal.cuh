@@ -163,6 +163,32 @@ __device__ void block_energy_add(long long *energy, int sys, const double (&v)[N
 
 struct SysDev;
 
+// Programmatic dependent launch, for chains of short kernels on one stream: a
+// kernel launched with launch_after may start as its predecessor's blocks end, and
+// calls wait_for_previous before it touches anything the predecessor writes or
+// reads.  Every block must call it, whatever else it does: the kernel after it
+// relies on this one having seen its predecessor's end.  A no-op for ordinary
+// launches.  (Predecessors do not let it start earlier: its waiting blocks would
+// hold SM slots of the pair kernel beside it.)  2,700 atoms 45.2 -> 44.6 us a step.
+__device__ __forceinline__ void wait_for_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... P, typename... A>
+cudaError_t launch_after(void (*kernel)(P...), int blocks, int threads, size_t smem,
+                         cudaStream_t stream, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // Component k of the FP64 minimum-image difference x_j - x_i, rounded to FP32.
 // The image is decided in FP32 where that is certain (|d| below 0.4999 L): one
 // FP64 subtraction and one conversion instead of five FP64-pipe operations.

@@ -24,6 +24,7 @@
 //              force accumulators.
 // Charges enter pre-scaled by sqrt(k_e), so the Coulomb constant needs no
 // extra multiply anywhere.
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -379,6 +380,7 @@ __global__ void __launch_bounds__(256) k_gather(PmeArgs a) {
         }
         goff = sd.grid_off;
     }
+    wait_for_previous();  // (the positions are older than the chain of transforms)
     int rel[3] = {0, 0, 0}, ex = 0, ey = 0, ez = 0;
     const int mode = a.tile_gather ? block_patch<P>(sp, active, sys, g, K, rel,
                                                     (long long)2 * kTilePerThread * blockDim.x,
@@ -709,12 +711,23 @@ cudaError_t launch_pme(mdg_system *s, int energy, int *cufft_status) {
         }
     }
     if (a.weight != 0.f) {  // weight 0: the energy alone
+        // behind this file's transforms alone: an ordinary launch waits for
+        // everything before it
+        const bool chained = std::all_of(p.groups.begin(), p.groups.end(),
+                                         [](const PmeGroup &g) { return g.own; });
+        auto gather = [&](auto kernel) -> cudaError_t {
+            if (chained) return launch_after(kernel, nb, ab, gather_smem, st, a);
+            kernel<<<nb, ab, gather_smem, st>>>(a);
+            return cudaGetLastError();
+        };
+        cudaError_t ge = cudaSuccess;
         switch (p.order) {
-            case 4: k_gather<4><<<nb, ab, gather_smem, st>>>(a); break;
-            case 5: k_gather<5><<<nb, ab, gather_smem, st>>>(a); break;
-            case 6: k_gather<6><<<nb, ab, gather_smem, st>>>(a); break;
+            case 4: ge = gather(k_gather<4>); break;
+            case 5: ge = gather(k_gather<5>); break;
+            case 6: ge = gather(k_gather<6>); break;
             default: break;
         }
+        if (ge != cudaSuccess) return ge;
         s->launches += 1;
     }
     return cudaGetLastError();

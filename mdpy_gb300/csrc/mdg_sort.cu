@@ -304,6 +304,7 @@ __global__ void k_partners_sorted(const int *__restrict__ perm, const int *__res
 // zeroing of the cluster's fixed-point force slots for the coming evaluation
 __global__ void k_pack(PackArgs a) {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    wait_for_previous();
     if (warp >= a.n_clusters) return;
     const int k = warp * kCluster + (threadIdx.x & 31);
     const int i = a.perm[k];
@@ -500,9 +501,9 @@ PackArgs make_pack_args(mdg_system *s) {
 
 cudaError_t launch_pack(mdg_system *s) {
     const int tb = 256;
-    k_pack<<<(s->n_clusters * 32 + tb - 1) / tb, tb, 0, s->stream>>>(make_pack_args(s));
     s->launches += 1;
-    return cudaGetLastError();
+    return launch_after(k_pack, (s->n_clusters * 32 + tb - 1) / tb, tb, 0, s->stream,
+                        make_pack_args(s));
 }
 
 }  // namespace mdg
