@@ -24,7 +24,7 @@ def _expected(orc, x, box, q, beta, K, order):
     return f, e, orc.ewald_self(q, beta) + orc.ewald_net_charge(q, box, beta)
 
 
-@pytest.mark.parametrize("order", [4, 6])
+@pytest.mark.parametrize("order", [4, 5, 6])
 def test_transforms_vs_oracle(lib, orc, order):
     grids = [g for g in GRIDS if min(g) >= 2 * order]
     systems = [_random(150 + 7 * k, K, k) for k, K in enumerate(grids)]
@@ -57,3 +57,29 @@ def test_transforms_vs_oracle(lib, orc, order):
         assert e[k, lib.TERM_COUL_RECIP] == pytest.approx(alone[k][1], rel=1e-6), grids[k]
         off += len(q)
     b.close()
+
+
+# a cluster and a bit, many clusters of a small system (8 atoms a warp), more
+# clusters (a thread per atom gathers), clusters unsplit in spreading
+@pytest.mark.parametrize("order", [4, 5, 6])
+@pytest.mark.parametrize("n,K", [(37, (12, 13, 18)), (3001, (30, 32, 36)), (45000, (64, 60, 72)),
+                                 (160000, (64, 60, 72))])
+def test_rows_equal_tiles(lib, order, n, K):
+    """Spreading and gathering row by row add the same contributions and read
+    the same values in the same order as through tiles (uncharged atoms and
+    partly filled clusters among them)."""
+    x, box, q = _random(n, K, n)
+    q[::5] = 0.0
+    s = lib.System(n, box)
+    s.set_charges(q)
+    s.nonbonded_config(2.0, 0.0, False, lib.COUL_EWALD, 0.35)
+    s.pme_config(K, order, 0.35)
+    s.set_positions(x)
+    out = []
+    for tiles in (0, 1, 2, 3):
+        s.set_launch_shape(4, 0, 64, 0, 1, tiles)
+        s.compute_forces(lib.mask(lib.TERM_COUL_RECIP))
+        out.append((s.get_forces(), s.get_energies()[0][lib.TERM_COUL_RECIP]))
+    for f, e in out[1:]:
+        assert np.array_equal(f, out[0][0]) and e == out[0][1]
+    s.close()
