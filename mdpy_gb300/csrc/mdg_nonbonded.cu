@@ -358,8 +358,9 @@ cudaError_t launch_nonbonded(mdg_system *s, unsigned mask, int energy, int dump)
     if (want_lj || coul_tile == MDG_COUL_EWALD) {
         // Ewald items of small systems, too few to fill the GPU, are taken by 8,
         // 4 or 2 warps each (the sums are the same).  Pair kernel alone, us at
-        // 1 / 2 / 4 / 8 warps: 416 items (2,700 atoms) 55 / 43 / 35 / 31, 900
-        // (6k atoms) 41 / 35 / 37 / 49; 1740 (12k) 67 / 67 / 68 / 103
+        // 1 / 2 / 4 / 8 warps: 404 items (2,700 atoms) 56 / 36 / 31 / 27, 516 (3,300)
+        // 41 / 29 / 25 / 26, 784 (5,100) 41 / 31 / 33 / 37, 1120 (7,800)
+        // 41 / 33 / 34 / 48
         const int warps = a.n_items <= 450 ? 8 : a.n_items <= 700 ? 4 : a.n_items <= 1200 ? 2 : 1;
         bool small = true;
         for (const SysDev &d : s->sys_h) small = small && d.n_atoms < kNbBlockSystem;

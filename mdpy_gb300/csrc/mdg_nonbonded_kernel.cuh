@@ -1372,45 +1372,47 @@ __global__ void __launch_bounds__(256, 2) k_nonbonded_block(NbArgs a) {
         return (unsigned)__cvta_generic_to_shared(ring + c * kPkChunk);
     };
     // Sweeps of the full super-chunks, one per warp in turn.  At the end of the
-    // scan a second pass takes the partial ones, merged and padded as the
-    // one-warp form does.
-    auto sweep_full = [&](bool last) {
-        for (int pass = 0; pass <= (last ? 1 : 0); ++pass) {
-            if (pass == 1) {
-                if (jcQ > 0 && jcL + jcQ <= 64) {
-                    if (w == 0)
-                        for (int k = lane; k < jcQ; k += 32)
-                            copy_entry_pk(ringQ, slot(bQ, k), ringL, slot(bL, jcL + k));
-                    jcL += jcQ;
-                    jcQ = 0;
-                }
-                auto pad = [&](float *ring, int b, int &jc, int warp) {
-                    if (jc == 0) return;
-                    if (w == warp)
-                        for (int k = jc + lane; k < 64; k += 32)
-                            put_entry_pk(ring, slot(b, k),
-                                         make_float4(kFarAway, kFarAway, kFarAway, 0.f),
-                                         make_float2(0.f, 0.f), kFull, -1);
-                    jc = 64;
-                };
-                pad(ringL, bL, jcL, 0);
-                pad(ringQ, bQ, jcQ, 1);
+    // scan the rests are merged and padded as the one-warp form does, and swept
+    // beside the full ones (in a pass of their own they took as long again).
+    auto sweep_full = [&](bool fin) {
+        __syncthreads();  // every entry is written
+        if (fin) {
+            const int rL = jcL & 63, rQ = jcQ & 63;
+            if (rQ > 0 && rL + rQ <= 64) {
+                if (w == 0)
+                    for (int k = lane; k < rQ; k += 32)
+                        copy_entry_pk(ringQ, slot(bQ, jcQ - rQ + k), ringL, slot(bL, jcL + k));
+                jcL += rQ;
+                jcQ -= rQ;
+                __syncwarp();
             }
-            __syncthreads();  // every entry is written
-            const int nL = jcL >> 6, nQ = jcQ >> 6;
-            for (int t = w; t < nL + nQ; t += W) {
-                const bool lj = t < nL;
-                const unsigned sa = lj ? addr(ringL, bL, t) : addr(ringQ, bQ, t - nL);
-                if (lj) sweep64<COUL, LJ, SWITCH, ENERGY, false, true>(a, sd, I2, pc, ik, lane, sa, S);
-                else sweep64<COUL, LJ, SWITCH, ENERGY, false, false>(a, sd, I2, pc, ik, lane, sa, S);
-                n_eval += 2048;
-            }
-            bL = bL + nL >= nc ? bL + nL - nc : bL + nL;
-            bQ = bQ + nQ >= nc ? bQ + nQ - nc : bQ + nQ;
-            jcL &= 63;
-            jcQ &= 63;
-            __syncthreads();  // the swept chunks may be overwritten
+            auto pad = [&](float *ring, int b, int &jc, int warp) {
+                const int up = (jc + 63) & ~63;
+                if (w == warp)
+                    for (int k = jc + lane; k < up; k += 32)
+                        put_entry_pk(ring, slot(b, k),
+                                     make_float4(kFarAway, kFarAway, kFarAway, 0.f),
+                                     make_float2(0.f, 0.f), kFull, -1);
+                jc = up;
+            };
+            pad(ringL, bL, jcL, 0);
+            pad(ringQ, bQ, jcQ, 1);
+            __syncthreads();
         }
+        const int nL = jcL >> 6, nQ = jcQ >> 6;
+        for (int t = w; t < nL + nQ; t += W) {
+            const bool lj = t < nL;
+            const unsigned sa = lj ? addr(ringL, bL, t) : addr(ringQ, bQ, t - nL);
+            if (lj) sweep64<COUL, LJ, SWITCH, ENERGY, false, true>(a, sd, I2, pc, ik, lane, sa, S);
+            else sweep64<COUL, LJ, SWITCH, ENERGY, false, false>(a, sd, I2, pc, ik, lane, sa, S);
+            n_eval += 2048;
+        }
+        if (fin) return;
+        bL = bL + nL >= nc ? bL + nL - nc : bL + nL;
+        bQ = bQ + nQ >= nc ? bQ + nQ - nc : bQ + nQ;
+        jcL &= 63;
+        jcQ &= 63;
+        __syncthreads();  // the swept chunks may be overwritten
     };
     int nh = 0, myJ = -1, mycode = 0;  // candidates of this round; this warp's
     auto candidate = [&](int J, int code) {
@@ -1474,9 +1476,16 @@ __global__ void __launch_bounds__(256, 2) k_nonbonded_block(NbArgs a) {
         jcQ += tQ;
         nh = 0;
         myJ = -1;
-        // a round's entries reach another warp's copy or padding only behind
-        // a barrier (the first pass of the last call has one)
-        if (last || max(jcL, jcQ) > cap - 32 * W) sweep_full(last);
+        // a round's entries reach another warp's copy or padding only behind the
+        // barrier that sweep_full begins with
+        if (last || max(jcL, jcQ) > cap - 32 * W) {
+            for (;;) {
+                // (merging may add a super-chunk to ring L)
+                const bool fin = last && max(jcL, jcQ) <= cap - 64;
+                sweep_full(fin);
+                if (fin || !last) break;
+            }
+        }
     };
     unsigned n_cand = 0;
     scan_candidates_one<ENERGY>(a, I, part, n_parts, sd, cI, hI, candidate, n_cand);
