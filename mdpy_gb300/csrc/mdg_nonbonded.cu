@@ -10,8 +10,9 @@
 // and adds the Ewald real-space term k q_i q_j erfc(beta r)/r (MDG_COUL_EWALD),
 // which mdpy v0.2.1 does not have, plus an optional CHARMM switch for LJ.
 //
-// Design (GB300): `split` (default 4) independent single-warp work items per 32-atom
-// i-cluster I (no block barrier: a warp that finishes early frees its slot).
+// Design (GB300): `split` (nb_default_parts) independent work items per 32-atom
+// i-cluster I, a warp each (no block barrier: a warp that finishes early frees its
+// slot); several warps each where items are few (the block form).
 //   1. each warp walks its own interleaved batches of cluster bounding boxes
 //      (a balanced half shell: the cluster pair {I, J} belongs to one of the
 //      two by the parity of I + J) and takes every (J, periodic image) whose
@@ -356,14 +357,28 @@ cudaError_t launch_nonbonded(mdg_system *s, unsigned mask, int energy, int dump)
     cudaError_t err = cudaSuccess;
     const int coul_tile = (want_c && s->coul_mode == MDG_COUL_EWALD) ? MDG_COUL_EWALD : MDG_COUL_NONE;
     if (want_lj || coul_tile == MDG_COUL_EWALD) {
-        // Ewald items of small systems, too few to fill the GPU, are taken by 8,
-        // 4 or 2 warps each (the sums are the same).  Pair kernel alone, us at
-        // 1 / 2 / 4 / 8 warps: 404 items (2,700 atoms) 56 / 36 / 31 / 27, 516 (3,300)
-        // 41 / 29 / 25 / 26, 784 (5,100) 41 / 31 / 33 / 37, 1120 (7,800)
-        // 41 / 33 / 34 / 48
-        const int warps = a.n_items <= 450 ? 8 : a.n_items <= 700 ? 4 : a.n_items <= 1200 ? 2 : 1;
+        // Ewald items of small systems, too few to fill the GPU, are taken by several
+        // warps each (the sums are the same): the most that keep every item with
+        // work resident (16 warps an SM at this kernel's registers; 4 warps less, as
+        // the PME and bonded kernels beside it take room).  A cluster's parts walk
+        // batches of 32 clusters, so a system of 64 to 96 has three parts with work.
+        // A whole step, us at 1 / 2 / 3 / 4 / 8 warps: 279 items with work (2,700 atoms,
+        // rc 12) 67 / 46 / 41 / 37 / 35, 408 (3,000, rc 9) 50 / 36 / 31 / 31 / 40, 536
+        // (3,900, rc 9) 49 / 36 / 33 / 33 / 45, 576 (4,200, rc 12) 57 / 41 / 37 / 40 / 50,
+        // 748 (5,400, rc 12) 80 / 56 / 52 / 55 / 65, 788 (5,700, rc 9) 50 / 38 / 45 / 48 / 57,
+        // 1060 (7,800, rc 10) 50 / 42 / 53 / 54 / 72
         bool small = true;
-        for (const SysDev &d : s->sys_h) small = small && d.n_atoms < kNbBlockSystem;
+        int work = 0;
+        for (const SysDev &d : s->sys_h) {
+            small = small && d.n_atoms < kNbBlockSystem;
+            const int cl = (d.n_atoms + kCluster - 1) / kCluster + d.n_cols / 2;
+            work += cl * std::min(a.split, (cl + 31) / 32);
+        }
+        const int warps = work <= 2 * s->n_sms        ? 8
+                          : work <= 18 * s->n_sms / 5 ? 4
+                          : work <= 5 * s->n_sms      ? 3
+                          : work <= 8 * s->n_sms      ? 2
+                                                      : 1;
         if (coul_tile == MDG_COUL_EWALD && s->nb_half == 0 && !s->nb_persistent && !dump && small &&
             warps > 1)
             err = launch_nb_block(s, a, warps, want_lj, sw, energy);

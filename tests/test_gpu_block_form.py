@@ -24,11 +24,11 @@ def _system(lib, ws, rc, switch, lj):
     return s
 
 
-# waters: eight warps an item, four, two (full scan, then columns), the largest
-# system of the form; a box of few clusters
+# waters: a box of few clusters; eight warps an item, four, two (full scan, then
+# columns), the largest system of the form; four by a full scan, three
 @pytest.mark.parametrize("n_waters,rc,switch,lj", [
     (40, 5.0, 0.0, True), (900, 12.0, 10.0, True), (1300, 9.0, 0.0, True), (2000, 10.0, 8.0, True),
-    (2600, 8.0, 0.0, False)])
+    (2600, 8.0, 0.0, False), (1000, 12.0, 10.0, True), (1700, 10.0, 0.0, True)])
 def test_block_form_equals_one_warp_form(lib, orc, n_waters, rc, switch, lj):
     from mdpy_gb300 import systems
 
