@@ -198,7 +198,7 @@ class NonbondedConstraint(CharmmNonbondedConstraint):
 
 
 class PMEConstraint(Constraint):
-    """Smooth particle-mesh Ewald reciprocal space (order-p B-splines, cuFFT),
+    """Smooth particle-mesh Ewald reciprocal space (order-p B-splines),
     plus the FP64 self and net-charge terms and the erf correction of the
     excluded pairs, so that NonbondedConstraint + PMEConstraint is the full
     Ewald sum.  ``grid_size`` defaults to the FFT-friendly size at

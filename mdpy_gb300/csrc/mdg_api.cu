@@ -6,11 +6,13 @@
 //   pack       FP32 cluster coordinates, bounding boxes, zeroed force slots
 //   nonbonded  LJ + Ewald real space (or LJ + bare Coulomb), half shell
 //   special    1-4 pairs and the Ewald exclusion correction
-//   pme        spread -> R2C -> convolve -> C2R -> gather
+//   pme        spread -> transforms and influence function -> gather
 //   bonded     bonds, angles, dihedrals, impropers
 // One MD step (Integrator.integrate, one step): pre-force update, force
-// evaluation, post-force update.  mdg_integrate replays chunks of
-// `reorder_interval` steps as one CUDA graph.
+// evaluation, post-force update (the latter and the next step's pre-force update
+// in one kernel inside a run).  mdg_integrate replays chunks of
+// `reorder_interval` steps as one CUDA graph, the steps before and after them as
+// graphs of one step; graphs are kept until what they froze changes.
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>

@@ -1,8 +1,8 @@
 """Integrators with mdpy's interface (mdpy/integrator/integrator.py:14-62).
 
 ``integrate(ensemble, num_steps)`` advances the device state; positions and
-velocities stay in HBM (FP64) and the steps run as CUDA-graph chunks inside
-libmdg.  One force evaluation per step.
+velocities stay in HBM (FP64) and the steps run as CUDA graphs inside libmdg,
+kept from one call to the next.  One force evaluation per step.
 
 * ``VerletIntegrator`` -- velocity Verlet.  mdpy's position-Verlet
   (mdpy/integrator/verlet_integrator.py:20-48) starts with a dt^2 instead of
