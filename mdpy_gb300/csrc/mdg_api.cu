@@ -235,8 +235,10 @@ int evaluate(mdg_system *s, unsigned mask, int energy) {
     if (!rc && e == cudaSuccess && lsp != kLsOff) e = ls_side(s, lsp);
     cudaError_t ej = cudaEventRecord(s->ev_join, s->side_stream);
     s->stream = s->bond_stream;
-    if (!rc && e == cudaSuccess && s->count_step) e = launch_count_step(s);
-    s->count_step = 0;
+    if (!rc && e == cudaSuccess && s->count_step) {
+        e = launch_count_step(s);
+        if (e == cudaSuccess) s->count_step = 0;
+    }
     if (!rc && e == cudaSuccess) e = launch_special(s, mask, energy, 0);
     if (!rc && e == cudaSuccess) e = launch_bonded(s, mask, energy);
     cudaError_t ej2 = cudaEventRecord(s->ev_join2, s->bond_stream);
@@ -286,6 +288,7 @@ int md_step(mdg_system *s, unsigned mask, StepEnd end) {
     CK(launch_move(s, pending), "integrate");
     s->count_step = pending ? 1 : 0;
     s->post_pending = 0;
+    s->forces_valid = 0;  // until the evaluation of the new positions is issued
     int rc;
     if (ls_active(s)) {
         rc = ls_evaluate(s, mask, energy, mts_weight(s, s->step) != 0.f ? kLsOuter : kLsInner);
@@ -298,9 +301,21 @@ int md_step(mdg_system *s, unsigned mask, StepEnd end) {
     if (rc) return rc;
     if (end != kMid) CK(launch_integrate_post(s, energy), "integrate post");
     else s->post_pending = 1;
+    s->forces_valid = 1;
     s->steps_since_reorder += 1;
     s->step += 1;
     return MDG_OK;
+}
+
+// What a run that an error ends may leave open, closed while the force buffer is
+// still that of its last finished step: the count of that step, whose kick was in
+// the first kernel of a step cut short, or its kick and count.  (Should these fail
+// as well, the next run still starts from the state the program sets.)
+void settle_run(mdg_system *s) {
+    if (s->count_step) (void)launch_count_step(s);
+    if (s->post_pending) (void)launch_integrate_post(s, 0);
+    s->count_step = 0;
+    s->post_pending = 0;
 }
 
 // Capture `nsteps` MD steps (the first re-sorting the atoms when `resort`, and
@@ -311,7 +326,7 @@ int capture_steps(mdg_system *s, Graph &g, int nsteps, int resort, unsigned mask
     const long long saved = s->launches;
     const int saved_since = s->steps_since_reorder, saved_need = s->need_reorder;
     const uint64_t saved_step = s->step;
-    const int saved_pending = s->post_pending;
+    const int saved_pending = s->post_pending, saved_valid = s->forces_valid;
     s->post_pending = pending;
     s->need_reorder = resort ? 1 : 0;
     if (!resort) s->steps_since_reorder = 0;
@@ -325,6 +340,8 @@ int capture_steps(mdg_system *s, Graph &g, int nsteps, int resort, unsigned mask
     s->need_reorder = saved_need;
     s->step = saved_step;
     s->post_pending = saved_pending;
+    s->forces_valid = saved_valid;
+    s->count_step = 0;
     const long long per = s->launches - saved;
     s->launches = saved;
     if (crc) {
@@ -1871,9 +1888,8 @@ MDG_API int mdg_set_step(mdg_system *s, uint64_t step) {
     return MDG_OK;
 }
 
-MDG_API int mdg_integrate(mdg_system *s, int n_steps, unsigned mask, int want_energy) {
-    int rc = check_sys(s);
-    if (rc) return rc;
+static int run_steps(mdg_system *s, int n_steps, unsigned mask, int want_energy) {
+    int rc = MDG_OK;
     if (n_steps < 0) return fail(MDG_ERR_INVALID, "negative step count");
     if (s->integ_kind < 0) return fail(MDG_ERR_STATE, "integrator has not been configured");
     mask &= MDG_MASK_ALL;
@@ -1887,12 +1903,6 @@ MDG_API int mdg_integrate(mdg_system *s, int n_steps, unsigned mask, int want_en
             for (auto &row : plane)
                 for (Graph &g : row)
                     if (g.exec && g.mask != mask) drop_step_graphs(s);
-    s->count_step = 0;
-    // a run that an error cut short: its last step's kick
-    if (s->post_pending) {
-        s->post_pending = 0;
-        CK(launch_integrate_post(s, 0), "integrate post");
-    }
     // the force buffer the first pre-force update uses: multiple time steps
     // want the weight of the evaluation that ended the previous step
     const float want_w = ls_active(s) ? -1.0f
@@ -1971,8 +1981,8 @@ MDG_API int mdg_integrate(mdg_system *s, int n_steps, unsigned mask, int want_en
         remaining -= 1;
     }
     if (s->post_pending) {  // the run ended with a chunk
-        s->post_pending = 0;
         CK(launch_integrate_post(s, 0), "integrate post");
+        s->post_pending = 0;
     }
     if (want_energy && n_steps == 0) {
         rc = evaluate(s, mask, 1);
@@ -1983,6 +1993,14 @@ MDG_API int mdg_integrate(mdg_system *s, int n_steps, unsigned mask, int want_en
     s->forces_mask = mask;
     CK(cudaGetLastError(), "integrate");
     return MDG_OK;
+}
+
+MDG_API int mdg_integrate(mdg_system *s, int n_steps, unsigned mask, int want_energy) {
+    int rc = check_sys(s);
+    if (rc) return rc;
+    rc = run_steps(s, n_steps, mask, want_energy);
+    if (rc) settle_run(s);
+    return rc;
 }
 
 MDG_API int mdg_pairset_dump(mdg_system *s, int32_t *pairs, int64_t capacity, int64_t *count) {

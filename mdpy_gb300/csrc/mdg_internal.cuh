@@ -641,7 +641,7 @@ struct mdg_system {
     unsigned forces_mask = 0;
     long long launches = 0;
     // Inside a run the kick that ends a step waits for the next step's first
-    // kernel (post_pending); a run ends with it done.
+    // kernel (post_pending); a run ends with it done, also one that an error ends.
     int post_pending = 0;
     int count_step = 0;                // the evaluation under way moves the step counter on
     mdg::Graph graph[2];               // chunk of reorder_interval steps: [kick pending]
