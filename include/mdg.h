@@ -370,7 +370,8 @@ MDG_API int mdg_integrator_config(mdg_system *sys, int kind, double dt, double t
                                   double friction, uint64_t seed);
 /* Integrator.integrate(ensemble, num_steps) (mdpy/integrator/integrator.py:24-27):
  * advances n_steps over the force terms in `mask`; energies of the final
- * step are evaluated when want_energy != 0.  Steps run as CUDA graphs. */
+ * step are evaluated when want_energy != 0.  Steps run as CUDA graphs, or launch by
+ * launch on a stream that the caller is capturing and on the legacy default stream. */
 MDG_API int mdg_integrate(mdg_system *sys, int n_steps, unsigned mask, int want_energy);
 /* current step counter (the Philox counter of the next step) */
 MDG_API int mdg_get_step(mdg_system *sys, uint64_t *step);

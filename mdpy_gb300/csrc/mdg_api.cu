@@ -389,11 +389,26 @@ int capture_eval(mdg_system *s, Graph &g, int resort, unsigned mask, int energy)
     return MDG_OK;
 }
 
+// Whether steps and evaluations may run as graphs of the library's own: not while the
+// caller is capturing the stream (they then become part of the caller's graph, launch
+// by launch), nor on the legacy default stream, which cannot be captured.
+int graphs_allowed(mdg_system *s, bool *yes) {
+    *yes = false;
+    if (s->stream == cudaStreamLegacy) return MDG_OK;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(s->stream, &st), "capture status");
+    *yes = st == cudaStreamCaptureStatusNone;
+    return MDG_OK;
+}
+
 // A force evaluation of the complete terms in `mask`: about 20 launches (30 with
 // a re-sort) of a few microseconds of host time each, so one that comes up again
 // is captured at its third run and replayed from then on (a capture costs about
 // what four eager runs do); always when `now`.
 int run_evaluation(mdg_system *s, unsigned mask, int energy, bool now) {
+    bool graphs = false;
+    if (const int rc = graphs_allowed(s, &graphs)) return rc;
+    if (!graphs) return evaluate(s, mask, energy);
     const int resort = s->need_reorder ? 1 : 0;
     Graph &g = s->graph_eval[energy ? 1 : 0][resort];
     if (g.mask != mask) {
@@ -1927,6 +1942,8 @@ static int run_steps(mdg_system *s, int n_steps, unsigned mask, int want_energy)
         s->forces_valid = 1;
         s->forces_mask = mask;
     }
+    bool graphs = false;
+    if ((rc = graphs_allowed(s, &graphs))) return rc;
     const int R = s->reorder_interval;
     int remaining = n_steps;
     while (remaining > 0) {
@@ -1934,7 +1951,7 @@ static int run_steps(mdg_system *s, int n_steps, unsigned mask, int want_energy)
         const int usable = remaining - (want_energy ? 1 : 0);
         // a whole chunk: one graph of R steps, captured when chunks keep coming
         // (it holds R times a step's 20 nodes), else R single steps
-        const bool whole = s->graph_mode == MDG_GRAPH_CHUNK && s->mts_k == 1 && chunk_start &&
+        const bool whole = graphs && s->graph_mode == MDG_GRAPH_CHUNK && s->mts_k == 1 && chunk_start &&
                            usable >= R && R >= 2;
         if (whole) s->chunk_uses += 1;
         Graph &gc = s->graph[s->post_pending];
@@ -1952,16 +1969,16 @@ static int run_steps(mdg_system *s, int n_steps, unsigned mask, int want_energy)
             remaining -= R;
             continue;
         }
-        // a single step: its kind's graph, captured at once in step mode and
+        // a single step: its kind's graph, if any, captured at once in step mode and
         // with multiple time steps; otherwise when it comes up again (a capture
         // costs about what four eager steps do)
         const StepEnd end = remaining > 1 ? kMid : want_energy ? kLastEnergy : kLast;
         const int outer = mts_weight(s, s->step) != 0.f ? 1 : 0;
         Graph &g = s->graph_step[s->post_pending][chunk_start ? 1 : 0][end][outer];
         const bool plain = !chunk_start && end == kMid && s->post_pending;
-        if (!g.exec && s->graph_mode == MDG_GRAPH_CHUNK && s->mts_k == 1 && g.uses < 2 &&
-            !(plain && remaining >= 6)) {
-            g.uses += 1;
+        if (!graphs || (!g.exec && s->graph_mode == MDG_GRAPH_CHUNK && s->mts_k == 1 &&
+                        g.uses < 2 && !(plain && remaining >= 6))) {
+            if (graphs) g.uses += 1;
             rc = md_step(s, mask, end);
             if (rc) return rc;
             remaining -= 1;

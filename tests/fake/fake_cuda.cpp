@@ -160,7 +160,8 @@ cudaError_t cudaGraphExecDestroy(cudaGraphExec_t e) {
 }
 }
 
-// a caller's own capture of a stream
+// a caller's own stream, and its capture
+FAKE_API void *fake_stream() { return new Stream(); }
 FAKE_API int fake_begin_capture(void *s) {
     return cudaStreamBeginCapture((cudaStream_t)s, cudaStreamCaptureModeRelaxed);
 }

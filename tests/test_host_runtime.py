@@ -1,5 +1,5 @@
 """libmdg's host side (mdg_api.cu) on a fake CUDA runtime: what a run leaves behind
-when one of its calls fails."""
+when one of its calls fails, and the streams that it takes."""
 import ctypes
 import os
 import subprocess
@@ -34,6 +34,7 @@ def fake_lib(tmp_path_factory):
     lib.fake_calls.argtypes = [ctypes.c_char_p]
     lib.fake_device_step.argtypes = [ctypes.c_void_p]
     lib.fake_device_step.restype = ctypes.c_longlong
+    lib.fake_stream.restype = ctypes.c_void_p
     lib.fake_begin_capture.argtypes = lib.fake_end_capture_and_run.argtypes = [ctypes.c_void_p]
     return lib
 
@@ -132,4 +133,54 @@ def test_a_step_cut_short_leaves_no_forces(fake):
         s.integrate(1, mask, want_energy=False)
     with pytest.raises(Exception, match="no force evaluation"):
         s.get_forces()
+    s.close()
+
+
+def _caller_stream(fake, kind):
+    if kind == "legacy":
+        return 0x1  # cudaStreamLegacy by its handle: cannot be captured
+    return fake.fake_stream()
+
+
+@pytest.mark.parametrize("kind", ["own", "legacy"])
+@pytest.mark.parametrize("step_mode", [False, True])
+@pytest.mark.parametrize("every", [1, 2])
+def test_runs_on_a_callers_stream(fake, kind, step_mode, every):
+    s, mask = _system()
+    s.set_graph_mode(1 if step_mode else 0)
+    s.set_mts(every)
+    s.set_stream(_caller_stream(fake, kind))
+    for _ in range(5):
+        s.compute_forces(mask)
+    done = 0
+    for n in (3, 9, 9, 9, 45, 250):
+        s.integrate(n, mask, want_energy=False)
+        done += n
+        _whole(fake, s, done)
+    assert (fake.fake_calls(b"cudaGraphLaunch") == 0) == (kind == "legacy")
+    s.close()
+
+
+@pytest.mark.parametrize("warm", [False, True])  # without and with graphs kept from before
+def test_work_under_a_callers_capture(fake, warm):
+    """Evaluations and runs on a stream that the caller is capturing become part of
+    the caller's graph, whatever the library would do with them otherwise."""
+    s, mask = _system()
+    stream = fake.fake_stream()
+    s.set_stream(stream)
+    if warm:
+        for _ in range(6):
+            s.compute_forces(mask)
+            s.integrate(9, mask, want_energy=False)
+        _restore(s)
+    assert fake.fake_begin_capture(stream) == 0
+    for _ in range(5):
+        s.compute_forces(mask)
+        s.integrate(9, mask, want_energy=False)
+    s.integrate(61, mask, want_energy=False)
+    assert fake.fake_device_step(s.handle) == 0  # nothing ran yet
+    assert fake.fake_end_capture_and_run(stream) == 0
+    _whole(fake, s, 106)
+    s.integrate(50, mask, want_energy=False)
+    _whole(fake, s, 156)
     s.close()
