@@ -164,21 +164,12 @@ int decode_status(mdg_system *s, int st) {
 }
 
 // The pinned staging words: the energy words of every system, the status word
-// (its low half) and one more.
+// (its low half) and one more.  Allocated with the system: a read allocates nothing.
 size_t stage_words(const mdg_system *s) { return (size_t)kEnergySlots * s->n_sys; }
-
-int stage_ready(mdg_system *s) {
-    if (!s->host_stage)
-        CK(cudaMallocHost((void **)&s->host_stage, sizeof(long long) * (stage_words(s) + 2)),
-           "pinned staging");
-    return MDG_OK;
-}
 
 // A read that ends with one synchronisation: the status word is copied beside
 // what is read (enqueue_status), and decoded after it (finish_status).
 int enqueue_status(mdg_system *s) {
-    const int rc = stage_ready(s);
-    if (rc) return rc;
     CK(cudaMemcpyAsync(s->host_stage + stage_words(s), s->status, sizeof(int),
                        cudaMemcpyDeviceToHost, s->stream),
        "status read");
@@ -525,6 +516,12 @@ MDG_API int mdg_system_create_batch(int device, int n_systems, const int *n_atom
     if (e != cudaSuccess) {
         mdg_system_destroy(s);
         return cuda_fail(e, "side stream");
+    }
+    e = cudaMallocHost((void **)&s->host_stage, sizeof(long long) * (stage_words(s) + 2));
+    if (e != cudaSuccess) {
+        s->host_stage = nullptr;
+        mdg_system_destroy(s);
+        return cuda_fail(e, "pinned staging");
     }
     const int n = s->n;
     int rc = MDG_OK;
@@ -1239,7 +1236,6 @@ MDG_API int mdg_kinetic_energy(mdg_system *s, double *kinetic) {
                          sizeof(long long), s->n_sys, s->stream),
        "memset");
     CK(launch_kinetic(s), "kinetic");
-    if ((rc = stage_ready(s))) return rc;
     const long long *e = s->host_stage;
     CK(cudaMemcpyAsync(s->host_stage, s->energy, sizeof(long long) * stage_words(s),
                        cudaMemcpyDeviceToHost, s->stream),
@@ -1505,11 +1501,9 @@ MDG_API int mdg_step_host(mdg_system *s, const double *x_in, const double *v_in,
     int rc = check_sys(s);
     if (rc) return rc;
     const size_t ne = (size_t)kEnergySlots * s->n_sys;
-    if (!s->host_stage || !s->xin || !s->same_flag) {
-        // pinned staging for the energy words, the status word and the
-        // positions-comparison flag; each buffer is allocated once, so a
-        // failed call leaves nothing half set up for the next one
-        if ((rc = stage_ready(s))) return rc;
+    if (!s->xin || !s->same_flag) {
+        // incoming positions and the comparison's flag; each buffer is allocated
+        // once, so a failed call leaves nothing half set up for the next one
         int rc2 = s->xin ? 0 : dalloc(&s->xin, 3 * (size_t)s->n);
         if (!rc2 && !s->same_flag) rc2 = dalloc(&s->same_flag, 1);
         if (rc2) return fail(rc2, "step_host staging");

@@ -184,3 +184,15 @@ def test_work_under_a_callers_capture(fake, warm):
     s.integrate(50, mask, want_energy=False)
     _whole(fake, s, 156)
     s.close()
+
+
+def test_reads_allocate_nothing(fake):
+    """Not even the first ones: a program may read while another thread captures, or
+    once its own pool holds the memory."""
+    s, mask = _system()
+    s.compute_forces(mask)
+    before = fake.fake_calls(b"cudaMalloc"), fake.fake_calls(b"cudaMallocHost")
+    s.get_positions(), s.get_velocities(), s.get_forces(), s.get_energies(), s.kinetic_energy()
+    s.check_status()
+    assert (fake.fake_calls(b"cudaMalloc"), fake.fake_calls(b"cudaMallocHost")) == before
+    s.close()
