@@ -486,12 +486,32 @@ __device__ __forceinline__ PkC pk_constants(const NbArgs &a) {
     return pc;
 }
 
+// A lane's sum of FP32 energies, exact to 2^-63: what a value keeps in units of 2^-32
+// in one word, the rest (less than half a unit, an exact difference) in another.  So
+// the order of the super-chunks and the split over warps do not matter, and an
+// item's total is rounded to 2^-32 once, as from an FP64 sum.  (One FP32 addition of
+// a super-chunk's halves and one rounding of it, 0 to 1.7 % faster with energies,
+// lost shares below half of 2^-32 and those beside a large one.)
+struct EnergySum {
+    long long hi = 0, lo = 0;  // units of 2^-32 and 2^-63
+    __device__ __forceinline__ void add(float v) {
+        const float t = v * kFixScaleF;
+        hi += __float2ll_rn(t);
+        lo += __float2int_rn((t - rintf(t)) * 2147483648.0f);
+    }
+    __device__ __forceinline__ void warp_sum() {
+        hi = warp_sum_ll(hi);
+        lo = warp_sum_ll(lo);
+    }
+    __device__ __forceinline__ long long total() const { return hi + ((lo + (1ll << 30)) >> 31); }
+};
+
 // A lane's i-force and energy sums over an item's super-chunks.
 // EWALD, systems below kNbBlockSystem: one FP32 sum per super-chunk, int64
 // fixed point across them, so the total does not depend on which warp swept
 // which super-chunk, nor on their order (the one-warp and the block form of the
 // kernel give the same bits).  Larger systems never use the block form: one
-// FP32 chain (a conversion per super-chunk costs 2 to 3 %).
+// FP32 chain (a conversion per super-chunk costs 2 to 3 %).  Energies: EnergySum.
 // Otherwise (LJ alone): one FP32 chain, energies in FP64.
 template <int COUL>
 struct ItemSums {
@@ -499,7 +519,7 @@ struct ItemSums {
     bool per_chunk = true;           // small system: the FP32 sums end with each super-chunk
     u64 FIX = 0ull, FIY = 0ull, FIZ = 0ull;  // +fr d, FP32
     long long fi[3] = {0, 0, 0};     // i force
-    long long e_lj = 0, e_c = 0;
+    EnergySum e_lj, e_c;
     // F: +fr d sums of the two packed halves
     __device__ __forceinline__ void add_force(const NbArgs &a, int axis, u64 F) {
         float p, q;
@@ -592,11 +612,15 @@ __device__ __forceinline__ void sweep64(const NbArgs &a, const SysDev &sd, const
         unpk2(CLJ, p0, p1);
         unpk2(CC, q0, q1);
         if constexpr (kFixed) {
-            const float el = p0 + p1, ec = q0 + q1;
-            if (!(fabsf(el) < kFixLimit && fabsf(ec) < kFixLimit))
+            if (!(fabsf(p0) < kFixLimit && fabsf(p1) < kFixLimit && fabsf(q0) < kFixLimit &&
+                  fabsf(q1) < kFixLimit))
                 raise_status(a.status, MDG_ERR_OVERFLOW);
-            S.e_lj += to_fix(el);
-            S.e_c += to_fix(ec);
+            if (LJ && WL) {  // (the charge-only sweeps have no LJ energy)
+                S.e_lj.add(p0);
+                S.e_lj.add(p1);
+            }
+            S.e_c.add(q0);
+            S.e_c.add(q1);
         } else {
             S.e_lj += (double)p0 + (double)p1;
             S.e_c += (double)q0 + (double)q1;
@@ -1300,8 +1324,10 @@ __device__ __forceinline__ void nb_item(const NbArgs &a, const int I, const int 
     if (ENERGY) {
         long long el, ee;  // fixed point
         if constexpr (!HALF && COUL == MDG_COUL_EWALD) {
-            el = warp_sum_ll(S.e_lj);
-            ee = warp_sum_ll(S.e_c);
+            S.e_lj.warp_sum();
+            S.e_c.warp_sum();
+            el = S.e_lj.total();
+            ee = S.e_c.total();
         } else {
             const double dl = warp_sum_d(acc_lj), dc = warp_sum_d(acc_c);
             if (lane == 0 && !(fabs(dl) < kFixLimit && fabs(dc) < kFixLimit))
@@ -1491,18 +1517,31 @@ __global__ void __launch_bounds__(256, 2) k_nonbonded_block(NbArgs a) {
 
     if (n_eval > 0 && xi.x < 0.5f * kFarAway) S.push_i(a, ik);
     if (ENERGY) {
+        // the item's energies in one total, rounded once
+        __shared__ EnergySum s_e[2][8];
         const unsigned n_in = __reduce_add_sync(kFull, S.n_in);
-        const long long el = warp_sum_ll(S.e_lj), ec = warp_sum_ll(S.e_c);
+        S.e_lj.warp_sum();
+        S.e_c.warp_sum();
         if (lane == 0) {
-            long long *es = a.energy + sid * kEnergySlots;
-            fix_red((unsigned long long *)&es[MDG_TERM_LJ], el);
-            fix_red((unsigned long long *)&es[MDG_TERM_COUL_REAL], ec);
+            s_e[0][w] = S.e_lj;
+            s_e[1][w] = S.e_c;
             atomicAdd(&a.stats[0], n_eval);
             atomicAdd(&a.stats[1], (unsigned long long)n_in);
             if (w == 0) {
                 atomicAdd(&a.stats[2], (unsigned long long)n_cand);
                 if (part == 0) atomicAdd(&a.stats[3], 1ull);
             }
+        }
+        __syncthreads();
+        if (threadIdx.x < 2) {
+            EnergySum e;
+            for (int k = 0; k < W; ++k) {
+                e.hi += s_e[threadIdx.x][k].hi;
+                e.lo += s_e[threadIdx.x][k].lo;
+            }
+            fix_red((unsigned long long *)&a.energy[sid * kEnergySlots + (threadIdx.x ? MDG_TERM_COUL_REAL
+                                                                                     : MDG_TERM_LJ)],
+                    e.total());
         }
     }
 }
