@@ -492,19 +492,36 @@ __device__ __forceinline__ PkC pk_constants(const NbArgs &a) {
 // item's total is rounded to 2^-32 once, as from an FP64 sum.  (One FP32 addition of
 // a super-chunk's halves and one rounding of it, 0 to 1.7 % faster with energies,
 // lost shares below half of 2^-32 and those beside a large one.)
+// The words wrap at 2^31 and are right all the same if the total is below: the FP32
+// sum beside them says whether it is.
 struct EnergySum {
     long long hi = 0, lo = 0;  // units of 2^-32 and 2^-63
+    float size = 0.f;
     __device__ __forceinline__ void add(float v) {
+        size += v;
         const float t = v * kFixScaleF;
         hi += __float2ll_rn(t);
         lo += __float2int_rn((t - rintf(t)) * 2147483648.0f);
     }
-    __device__ __forceinline__ void warp_sum() {
-        hi = warp_sum_ll(hi);
-        lo = warp_sum_ll(lo);
-    }
-    __device__ __forceinline__ long long total() const { return hi + ((lo + (1ll << 30)) >> 31); }
 };
+// What an item's lanes add up to (of one warp, or of several).
+struct EnergyTotal {
+    long long hi, lo;
+    float size;
+    __device__ __forceinline__ long long fixed(int *status) const {
+        if (!(fabsf(size) < kFixLimit)) raise_status(status, MDG_ERR_OVERFLOW);
+        return hi + ((lo + (1ll << 30)) >> 31);
+    }
+};
+__device__ __forceinline__ EnergyTotal warp_total(const EnergySum &e) {
+    EnergyTotal t;
+    t.hi = warp_sum_ll(e.hi);
+    t.lo = warp_sum_ll(e.lo);
+    t.size = e.size;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t.size += __shfl_xor_sync(kFull, t.size, o);
+    return t;
+}
 
 // A lane's i-force and energy sums over an item's super-chunks.
 // EWALD, systems below kNbBlockSystem: one FP32 sum per super-chunk, int64
@@ -612,8 +629,8 @@ __device__ __forceinline__ void sweep64(const NbArgs &a, const SysDev &sd, const
         unpk2(CLJ, p0, p1);
         unpk2(CC, q0, q1);
         if constexpr (kFixed) {
-            if (!(fabsf(p0) < kFixLimit && fabsf(p1) < kFixLimit && fabsf(q0) < kFixLimit &&
-                  fabsf(q1) < kFixLimit))
+            // what does not convert (a NaN shows in the total's size)
+            if (!(fmaxf(fmaxf(fabsf(p0), fabsf(p1)), fmaxf(fabsf(q0), fabsf(q1))) < 2147483648.0f))
                 raise_status(a.status, MDG_ERR_OVERFLOW);
             if (LJ && WL) {  // (the charge-only sweeps have no LJ energy)
                 S.e_lj.add(p0);
@@ -1322,12 +1339,13 @@ __device__ __forceinline__ void nb_item(const NbArgs &a, const int I, const int 
         fix_red(&a.f[2 * a.n_pad + ik], to_fix(fiz));
     }
     if (ENERGY) {
-        long long el, ee;  // fixed point
+        long long el = 0, ee = 0;  // fixed point, in lane 0
         if constexpr (!HALF && COUL == MDG_COUL_EWALD) {
-            S.e_lj.warp_sum();
-            S.e_c.warp_sum();
-            el = S.e_lj.total();
-            ee = S.e_c.total();
+            const EnergyTotal tl = warp_total(S.e_lj), tc = warp_total(S.e_c);
+            if (lane == 0) {
+                el = tl.fixed(a.status);
+                ee = tc.fixed(a.status);
+            }
         } else {
             const double dl = warp_sum_d(acc_lj), dc = warp_sum_d(acc_c);
             if (lane == 0 && !(fabs(dl) < kFixLimit && fabs(dc) < kFixLimit))
@@ -1518,13 +1536,12 @@ __global__ void __launch_bounds__(256, 2) k_nonbonded_block(NbArgs a) {
     if (n_eval > 0 && xi.x < 0.5f * kFarAway) S.push_i(a, ik);
     if (ENERGY) {
         // the item's energies in one total, rounded once
-        __shared__ EnergySum s_e[2][8];
+        __shared__ EnergyTotal s_e[2][8];
         const unsigned n_in = __reduce_add_sync(kFull, S.n_in);
-        S.e_lj.warp_sum();
-        S.e_c.warp_sum();
+        const EnergyTotal tl = warp_total(S.e_lj), tc = warp_total(S.e_c);
         if (lane == 0) {
-            s_e[0][w] = S.e_lj;
-            s_e[1][w] = S.e_c;
+            s_e[0][w] = tl;
+            s_e[1][w] = tc;
             atomicAdd(&a.stats[0], n_eval);
             atomicAdd(&a.stats[1], (unsigned long long)n_in);
             if (w == 0) {
@@ -1534,14 +1551,15 @@ __global__ void __launch_bounds__(256, 2) k_nonbonded_block(NbArgs a) {
         }
         __syncthreads();
         if (threadIdx.x < 2) {
-            EnergySum e;
-            for (int k = 0; k < W; ++k) {
+            EnergyTotal e = s_e[threadIdx.x][0];
+            for (int k = 1; k < W; ++k) {
                 e.hi += s_e[threadIdx.x][k].hi;
                 e.lo += s_e[threadIdx.x][k].lo;
+                e.size += s_e[threadIdx.x][k].size;
             }
             fix_red((unsigned long long *)&a.energy[sid * kEnergySlots + (threadIdx.x ? MDG_TERM_COUL_REAL
                                                                                      : MDG_TERM_LJ)],
-                    e.total());
+                    e.fixed(a.status));
         }
     }
 }

@@ -79,3 +79,23 @@ def test_a_small_share_beside_a_large_one(lib, n, many):
     share = sum(unit.COULOMB_K * 1000.0 * 1e-3 * math.erfc(BETA * r) / r for r in (6.0, 5.5))
     # FP32 pair arithmetic 1e-5, one rounding to 2^-32 an item in each run
     assert abs(energies[1] - energies[0] - share) <= 1e-5 * share + 8 * 2.0 ** -33
+
+
+@pytest.mark.parametrize("n,many,items", [(64, False, 5), (64, True, 5), (9000, False, 1200)])
+def test_an_item_beyond_the_range_is_refused(lib, orc, n, many, items):
+    """Like charges whose energies make an item's total pass 1e9 (what int64 fixed point
+    holds, with room), although no lane's share and no force does; half of that
+    in the whole system is taken, and right."""
+    edge = 20.0 if n == 64 else (n / 0.1) ** (1 / 3)
+    x, rc = _lattice(n, edge, 3), 9.0
+    none = np.full((n, 1), -1)
+    unit_energy = orc.nonbonded(x, np.full(3, edge), np.zeros((n, 4)), np.ones(n), none, none, rc,
+                                lj=False, coulomb="ewald", beta=BETA)[1]["coulomb"]
+
+    def energy(total):
+        q = np.full(n, math.sqrt(total / unit_energy))
+        return _energy(lib, [(x, q, np.full(3, edge))] + _fillers(many), 0, rc)[0]
+
+    with pytest.raises(Exception, match="fixed-point range"):
+        energy(items * 2.5e9)
+    assert energy(5e8) == pytest.approx(5e8, rel=1e-5)
