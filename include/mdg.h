@@ -210,9 +210,9 @@ MDG_API int mdg_step_host(mdg_system *sys, const double *x_in, const double *v_i
 /* ---- launch shapes and the autotuner (no reference counterpart) ---------
  * A launch shape is MDG_SHAPE_FIELDS ints:
  *   [MDG_SHAPE_SPLIT]          work items (one warp each) per 32-atom cluster in
- *                              the pair kernel: 1, 2, 4, 8, 16 (default: 4; with
- *                              Ewald 2 for each system of 128,000 atoms or more).
- *                              Few items of small systems are taken by several
+ *                              the pair kernel: 1, 2, 4, 8, 16, or 0 (default): by
+ *                              the size of each system, 4, and with Ewald 2 from
+ *                              128,000 atoms on.  Few items of small systems are taken by several
  *                              warps each, with the same sums;
  *   [MDG_SHAPE_PERSISTENT]     0 = one CTA per work item; n = n resident CTAs
  *                              per SM (1..24) pulling work items from a device
@@ -250,7 +250,8 @@ MDG_API int mdg_get_launch_shape(mdg_system *sys, int *shape);
  * `mask`.  Phase one varies the pair kernel (split 2/4/8 x persistent 0/20/24
  * x split rings 0/1 x half 0/1/2), phase two PME and the streams (block 64/128/256 x tiles
  * 0-3 x side priority 0/1) around phase one's best; then the four fastest and
- * the shape in use are re-timed, interleaved, over 4 x reps and the fastest
+ * the shape in use (a split by size as the number it stands for, where it is one for
+ * all systems) are re-timed, interleaved, over 4 x reps and the fastest
  * is kept; *best_ms (may be NULL) receives its time.  Leaves no valid force
  * evaluation. */
 MDG_API int mdg_autotune(mdg_system *sys, unsigned mask, int reps, double *best_ms);

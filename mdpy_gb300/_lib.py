@@ -350,9 +350,10 @@ class System:
     SHAPE_FIELDS = ("split", "persistent", "pme_block", "side_priority", "split_rings",
                     "pme_tiles", "half")
 
-    def set_launch_shape(self, split=4, persistent=0, pme_block=256, side_priority=0,
+    def set_launch_shape(self, split=0, persistent=0, pme_block=256, side_priority=0,
                          split_rings=1, pme_tiles=0, half=0):
-        """``persistent``: 0 = one CTA per pair work item, n = n resident CTAs
+        """``split``: work items per cluster of the pair kernel, 0 = by the size
+        of each system; ``persistent``: 0 = one CTA per pair work item, n = n resident CTAs
         per SM pulling work items; ``pme_tiles``: bit 0 tiled spreading, bit 1
         tiled gathering; ``half``: 16-atom i groups per half warp."""
         sh = (ctypes.c_int * 7)(int(split), int(persistent), int(pme_block), int(side_priority),

@@ -1281,8 +1281,8 @@ static int apply_shape(mdg_system *s, const int *sh) {
               pme_block = sh[MDG_SHAPE_PME_BLOCK], side_priority = sh[MDG_SHAPE_SIDE_PRIORITY],
               split_rings = sh[MDG_SHAPE_SPLIT_RINGS], pme_tiles = sh[MDG_SHAPE_PME_TILES],
               half = sh[MDG_SHAPE_HALF];
-    if (split != 1 && split != 2 && split != 4 && split != 8 && split != 16)
-        return fail(MDG_ERR_INVALID, "split %d is not 1, 2, 4, 8 or 16", split);
+    if (split != 0 && split != 1 && split != 2 && split != 4 && split != 8 && split != 16)
+        return fail(MDG_ERR_INVALID, "split %d is not 0, 1, 2, 4, 8 or 16", split);
     if (persistent < 0 || persistent > 24)
         return fail(MDG_ERR_INVALID, "persistent CTAs per SM %d not in 0..24", persistent);
     if (pme_block != 64 && pme_block != 128 && pme_block != 256)
@@ -1310,7 +1310,7 @@ static int apply_shape(mdg_system *s, const int *sh) {
 }
 
 static void current_shape(const mdg_system *s, int *sh) {
-    sh[MDG_SHAPE_SPLIT] = nb_parts(s);
+    sh[MDG_SHAPE_SPLIT] = s->nb_split;
     sh[MDG_SHAPE_PERSISTENT] = s->nb_persistent;
     sh[MDG_SHAPE_PME_BLOCK] = s->pme_block;
     sh[MDG_SHAPE_SIDE_PRIORITY] = s->side_priority;
@@ -1408,9 +1408,13 @@ MDG_API int mdg_autotune(mdg_system *s, unsigned mask, int reps, double *best_ms
         return r;
     };
     auto by_time = [](const Shape &x, const Shape &y) { return x.ms < y.ms; };
-    Shape current;
-    current_shape(s, current.sh);
-    current.ms = 0.f;
+    Shape initial, current;
+    current_shape(s, initial.sh);
+    initial.ms = 0.f;
+    current = initial;
+    // by size, with one number for all systems: that number, as the others tried
+    if (current.sh[MDG_SHAPE_SPLIT] == 0 && nb_parts_uniform(s))
+        current.sh[MDG_SHAPE_SPLIT] = nb_parts(s);
     const bool pme = (mask & MDG_MASK(MDG_TERM_COUL_RECIP)) && s->pme.on;
     std::vector<Shape> tried;
     // phase one: the pair kernel
@@ -1441,7 +1445,7 @@ MDG_API int mdg_autotune(mdg_system *s, unsigned mask, int reps, double *best_ms
                     tried.push_back(c);
                 }
     }
-    Shape best = current;
+    Shape best = initial;
     float best_t = 0.f;
     if (!rc && ce == cudaSuccess) {
         std::sort(tried.begin(), tried.end(), by_time);

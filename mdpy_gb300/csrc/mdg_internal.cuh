@@ -664,7 +664,8 @@ cudaError_t launch_reorder(mdg_system *s);
 cudaError_t launch_pack(mdg_system *s);
 PackArgs make_pack_args(mdg_system *s);
 cudaError_t launch_nonbonded(mdg_system *s, unsigned mask, int energy, int dump);
-int nb_parts(const mdg_system *s);  // work items per cluster of the pair kernel
+int nb_parts(const mdg_system *s);  // work items per cluster of the pair kernel, at most
+bool nb_parts_uniform(const mdg_system *s);  // and of every system
 cudaError_t launch_special(mdg_system *s, unsigned mask, int energy, int dump);
 cudaError_t launch_pme(mdg_system *s, int energy, int *cufft_status);
 cudaError_t launch_bonded(mdg_system *s, unsigned mask, int energy);

@@ -339,6 +339,13 @@ int nb_parts(const mdg_system *s) {
     return p;
 }
 
+bool nb_parts_uniform(const mdg_system *s) {
+    if (s->nb_split > 0 || s->coul_mode != MDG_COUL_EWALD) return true;
+    const int p = nb_default_parts(s->sys_h[0].n_atoms);
+    return std::all_of(s->sys_h.begin(), s->sys_h.end(),
+                       [p](const SysDev &d) { return nb_default_parts(d.n_atoms) == p; });
+}
+
 cudaError_t launch_nonbonded(mdg_system *s, unsigned mask, int energy, int dump) {
     const bool want_lj = (mask & MDG_MASK(MDG_TERM_LJ)) && s->lj_on;
     const bool want_c = (mask & MDG_MASK(MDG_TERM_COUL_REAL)) && s->coul_mode != MDG_COUL_NONE;

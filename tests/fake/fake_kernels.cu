@@ -31,6 +31,7 @@ cudaError_t launch_nonbonded(mdg_system *s, unsigned, int energy, int) {
     });
 }
 int nb_parts(const mdg_system *) { return 4; }
+bool nb_parts_uniform(const mdg_system *) { return true; }
 cudaError_t launch_special(mdg_system *, unsigned, int, int) { return issue("special", [] {}); }
 cudaError_t launch_pme(mdg_system *, int, int *) { return issue("pme", [] {}); }
 cudaError_t launch_bonded(mdg_system *, unsigned, int) { return issue("bonded", [] {}); }

@@ -196,3 +196,18 @@ def test_reads_allocate_nothing(fake):
     s.check_status()
     assert (fake.fake_calls(b"cudaMalloc"), fake.fake_calls(b"cudaMallocHost")) == before
     s.close()
+
+
+def test_a_launch_shape_can_be_read_and_written_back(fake):
+    s, _ = _system()
+    default = s.launch_shape
+    assert default["split"] == 0  # by the size of each system
+    s.set_launch_shape(split=8, pme_block=64)
+    assert s.launch_shape["split"] == 8
+    s.set_launch_shape(**default)
+    assert s.launch_shape == default
+    s.set_launch_shape(pme_block=128)
+    assert s.launch_shape == dict(default, pme_block=128)
+    with pytest.raises(Exception, match="split"):
+        s.set_launch_shape(split=3)
+    s.close()
