@@ -46,9 +46,9 @@ cudaError_t launch_nb_quarter(mdg_system *s, const NbArgs &a, int coul_tile, boo
                               bool sw, int energy, int dump);  // mdg_nonbonded_quarter.cu
 
 cudaError_t launch_nb_batch(mdg_system *s, const NbArgs &a, int coul_tile, bool want_lj, bool sw,
-                            int energy);  // mdg_nonbonded_batch.cu
+                            int energy, int dump);  // mdg_nonbonded_batch.cu
 cudaError_t launch_nb_block(mdg_system *s, const NbArgs &a, int warps, bool want_lj, bool sw,
-                            int energy);  // mdg_nonbonded_block.cu
+                            int energy, int dump);  // mdg_nonbonded_block.cu
 
 namespace {
 
@@ -386,15 +386,17 @@ cudaError_t launch_nonbonded(mdg_system *s, unsigned mask, int energy, int dump)
                           : work <= 5 * s->n_sms      ? 3
                           : work <= 8 * s->n_sms      ? 2
                                                       : 1;
-        if (coul_tile == MDG_COUL_EWALD && s->nb_half == 0 && !s->nb_persistent && !dump && small &&
-            warps > 1)
-            err = launch_nb_block(s, a, warps, want_lj, sw, energy);
+        // (a pair dump takes the form that the system's forces take: it asks for LJ
+        // alone, so the mode decides)
+        const bool ewald = dump ? s->coul_mode == MDG_COUL_EWALD : coul_tile == MDG_COUL_EWALD;
+        if (ewald && s->nb_half == 0 && !s->nb_persistent && small && warps > 1)
+            err = launch_nb_block(s, a, warps, want_lj, sw, energy, dump);
         else
             err = s->nb_half == 2   ? launch_nb_quarter(s, a, coul_tile, want_lj, sw, energy, dump)
                   : s->nb_half == 1 ? launch_nb_half(s, a, coul_tile, want_lj, sw, energy, dump)
-                  : (s->n_sys > 1 || small) && !dump
-                      ? launch_nb_batch(s, a, coul_tile, want_lj, sw, energy)
-                                    : dispatch_shape<false>(s, a, coul_tile, want_lj, sw, energy, dump);
+                  : s->n_sys > 1 || small
+                      ? launch_nb_batch(s, a, coul_tile, want_lj, sw, energy, dump)
+                      : dispatch_shape<false>(s, a, coul_tile, want_lj, sw, energy, dump);
         s->launches += 1;
         if (err != cudaSuccess) return err;
     }

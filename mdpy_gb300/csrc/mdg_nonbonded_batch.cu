@@ -6,8 +6,8 @@
 namespace mdg {
 
 cudaError_t launch_nb_batch(mdg_system *s, const NbArgs &a, int coul_tile, bool want_lj, bool sw,
-                            int energy) {
-    return dispatch_shape<false, true>(s, a, coul_tile, want_lj, sw, energy, 0);
+                            int energy, int dump) {
+    return dispatch_shape<false, true>(s, a, coul_tile, want_lj, sw, energy, dump);
 }
 
 }  // namespace mdg

@@ -1020,9 +1020,8 @@ __device__ __forceinline__ void nb_item(const NbArgs &a, const int I, const int 
     // this cluster's system and its box
     const int sid = a.cl_sys[I];
     const SysDev &sd = a.sys[sid];
-    // the whole-warp form with five sites only takes one system, or a pair dump:
-    // a.split is its parts, a constant to its scan loops (88k atoms 242 -> 239 us,
-    // 500k 1092 -> 1080)
+    // the whole-warp form with five sites only takes one system: a.split is its
+    // parts, a constant to its scan loops (88k atoms 242 -> 239 us, 500k 1092 -> 1080)
     const int n_parts = ONE || HALF ? item_parts(a, sd) : a.split;
     if (part >= n_parts) return;
     const float L[3] = {sd.L[0], sd.L[1], sd.L[2]};
@@ -1381,7 +1380,7 @@ __device__ __forceinline__ void nb_item(const NbArgs &a, const int I, const int 
 // and W warps' worth of sweeps between rounds
 __host__ __device__ constexpr int nb_block_chunks(int warps) { return warps == 8 ? 8 : warps == 4 ? 6 : 5; }
 
-template <int COUL, bool LJ, bool SWITCH, bool ENERGY>
+template <int COUL, bool LJ, bool SWITCH, bool ENERGY, bool DUMP>
 __global__ void __launch_bounds__(256, 2) k_nonbonded_block(NbArgs a) {
     extern __shared__ __align__(2048) float s_rings[];
     __shared__ int2 s_cnt[2][8];
@@ -1446,8 +1445,8 @@ __global__ void __launch_bounds__(256, 2) k_nonbonded_block(NbArgs a) {
         for (int t = w; t < nL + nQ; t += W) {
             const bool lj = t < nL;
             const unsigned sa = lj ? addr(ringL, bL, t) : addr(ringQ, bQ, t - nL);
-            if (lj) sweep64<COUL, LJ, SWITCH, ENERGY, false, true>(a, sd, I2, pc, ik, lane, sa, S);
-            else sweep64<COUL, LJ, SWITCH, ENERGY, false, false>(a, sd, I2, pc, ik, lane, sa, S);
+            if (lj) sweep64<COUL, LJ, SWITCH, ENERGY, DUMP, true>(a, sd, I2, pc, ik, lane, sa, S);
+            else sweep64<COUL, LJ, SWITCH, ENERGY, DUMP, false>(a, sd, I2, pc, ik, lane, sa, S);
             n_eval += 2048;
         }
         if (fin) return;
@@ -1533,7 +1532,7 @@ __global__ void __launch_bounds__(256, 2) k_nonbonded_block(NbArgs a) {
     unsigned n_cand = 0;
     scan_candidates_one<ENERGY>(a, I, part, n_parts, sd, cI, hI, candidate, n_cand);
 
-    if (n_eval > 0 && xi.x < 0.5f * kFarAway) S.push_i(a, ik);
+    if (!DUMP && n_eval > 0 && xi.x < 0.5f * kFarAway) S.push_i(a, ik);
     if (ENERGY) {
         // the item's energies in one total, rounded once
         __shared__ EnergyTotal s_e[2][8];
@@ -1867,7 +1866,7 @@ cudaError_t dispatch_nb(mdg_system *s, const NbArgs &a, int energy, int dump) {
     if (a.persistent && cudaMemsetAsync(a.queue, 0, sizeof(int), s->stream) != cudaSuccess)
         return cudaGetLastError();
     if (dump) {
-        if constexpr (COUL == MDG_COUL_EWALD && LJ && !SW && !ONE)
+        if constexpr (COUL == MDG_COUL_EWALD && LJ && !SW)
             k_nonbonded<COUL, LJ, SW, false, true, HALF, ONE><<<grid, block, 0, s->stream>>>(a);
     } else if (energy)
         k_nonbonded<COUL, LJ, SW, true, false, HALF, ONE><<<grid, block, 0, s->stream>>>(a);
