@@ -380,15 +380,22 @@ int capture_eval(mdg_system *s, Graph &g, int resort, unsigned mask, int energy)
     return MDG_OK;
 }
 
-// Whether steps and evaluations may run as graphs of the library's own: not while the
-// caller is capturing the stream (they then become part of the caller's graph, launch
-// by launch), nor on the legacy default stream, which cannot be captured.
-int graphs_allowed(mdg_system *s, bool *yes) {
-    *yes = false;
+// Which work may run as graphs of the library's own.  None while the caller is capturing
+// the stream (it then becomes part of the caller's graph, launch by launch), nor on
+// the legacy default stream, which cannot be captured.  On a stream that synchronises
+// with the legacy one only what asks for graphs (whole chunks, step mode, multiple
+// time steps): while it is being captured, other threads' work on the legacy stream
+// fails, so that evaluations and short runs leave it alone.
+enum GraphUse { kNoGraphs, kAskedFor, kAnyWork };
+int graph_use(mdg_system *s, GraphUse *use) {
+    *use = kNoGraphs;
     if (s->stream == cudaStreamLegacy) return MDG_OK;
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(s->stream, &st), "capture status");
-    *yes = st == cudaStreamCaptureStatusNone;
+    if (st != cudaStreamCaptureStatusNone) return MDG_OK;
+    unsigned flags = 0;
+    CK(cudaStreamGetFlags(s->stream, &flags), "stream flags");
+    *use = flags & cudaStreamNonBlocking ? kAnyWork : kAskedFor;
     return MDG_OK;
 }
 
@@ -397,9 +404,9 @@ int graphs_allowed(mdg_system *s, bool *yes) {
 // is captured at its third run and replayed from then on (a capture costs about
 // what four eager runs do); always when `now`.
 int run_evaluation(mdg_system *s, unsigned mask, int energy, bool now) {
-    bool graphs = false;
-    if (const int rc = graphs_allowed(s, &graphs)) return rc;
-    if (!graphs) return evaluate(s, mask, energy);
+    GraphUse use;
+    if (const int rc = graph_use(s, &use)) return rc;
+    if (use == kNoGraphs || (use == kAskedFor && !now)) return evaluate(s, mask, energy);
     const int resort = s->need_reorder ? 1 : 0;
     Graph &g = s->graph_eval[energy ? 1 : 0][resort];
     if (g.mask != mask) {
@@ -1940,8 +1947,10 @@ static int run_steps(mdg_system *s, int n_steps, unsigned mask, int want_energy)
         s->forces_valid = 1;
         s->forces_mask = mask;
     }
-    bool graphs = false;
-    if ((rc = graphs_allowed(s, &graphs))) return rc;
+    GraphUse use;
+    if ((rc = graph_use(s, &use))) return rc;
+    const bool asked = s->graph_mode == MDG_GRAPH_STEP || s->mts_k > 1;
+    const bool graphs = use == kAnyWork || (use == kAskedFor && asked);  // of single steps
     const int R = s->reorder_interval;
     int remaining = n_steps;
     while (remaining > 0) {
@@ -1949,7 +1958,7 @@ static int run_steps(mdg_system *s, int n_steps, unsigned mask, int want_energy)
         const int usable = remaining - (want_energy ? 1 : 0);
         // a whole chunk: one graph of R steps, captured when chunks keep coming
         // (it holds R times a step's 20 nodes), else R single steps
-        const bool whole = graphs && s->graph_mode == MDG_GRAPH_CHUNK && s->mts_k == 1 && chunk_start &&
+        const bool whole = use != kNoGraphs && s->graph_mode == MDG_GRAPH_CHUNK && s->mts_k == 1 && chunk_start &&
                            usable >= R && R >= 2;
         if (whole) s->chunk_uses += 1;
         Graph &gc = s->graph[s->post_pending];
@@ -1974,8 +1983,8 @@ static int run_steps(mdg_system *s, int n_steps, unsigned mask, int want_energy)
         const int outer = mts_weight(s, s->step) != 0.f ? 1 : 0;
         Graph &g = s->graph_step[s->post_pending][chunk_start ? 1 : 0][end][outer];
         const bool plain = !chunk_start && end == kMid && s->post_pending;
-        if (!graphs || (!g.exec && s->graph_mode == MDG_GRAPH_CHUNK && s->mts_k == 1 &&
-                        g.uses < 2 && !(plain && remaining >= 6))) {
+        if (!graphs ||
+            (!g.exec && !asked && g.uses < 2 && !(plain && remaining >= 6))) {
             if (graphs) g.uses += 1;
             rc = md_step(s, mask, end);
             if (rc) return rc;

@@ -14,7 +14,9 @@
 namespace {
 
 using Op = std::function<void()>;
-struct Stream {};
+struct Stream {
+    unsigned flags = 0;
+};
 std::vector<Op> *capture = nullptr;  // the graph being captured, if any
 cudaStream_t capturing = nullptr;    // and the stream that began it
 std::map<std::string, int> calls, fail_at;
@@ -95,12 +97,15 @@ cudaError_t cudaMemset2DAsync(void *d, size_t pitch, int v, size_t w, size_t h, 
         for (size_t r = 0; r < h; ++r) memset((char *)d + r * pitch, v, w);
     });
 }
-cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
-    *s = (cudaStream_t) new Stream();
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned flags) {
+    *s = (cudaStream_t) new Stream{flags};
     return cudaSuccess;
 }
-cudaError_t cudaStreamCreateWithPriority(cudaStream_t *s, unsigned, int) {
-    *s = (cudaStream_t) new Stream();
+cudaError_t cudaStreamCreateWithPriority(cudaStream_t *s, unsigned flags, int) {
+    return cudaStreamCreateWithFlags(s, flags);
+}
+cudaError_t cudaStreamGetFlags(cudaStream_t s, unsigned *flags) {
+    *flags = ((Stream *)s)->flags;
     return cudaSuccess;
 }
 cudaError_t cudaStreamDestroy(cudaStream_t s) {
@@ -161,7 +166,7 @@ cudaError_t cudaGraphExecDestroy(cudaGraphExec_t e) {
 }
 
 // a caller's own stream, and its capture
-FAKE_API void *fake_stream() { return new Stream(); }
+FAKE_API void *fake_stream(unsigned flags) { return new Stream{flags}; }
 FAKE_API int fake_begin_capture(void *s) {
     return cudaStreamBeginCapture((cudaStream_t)s, cudaStreamCaptureModeRelaxed);
 }

@@ -34,7 +34,7 @@ def fake_lib(tmp_path_factory):
     lib.fake_calls.argtypes = [ctypes.c_char_p]
     lib.fake_device_step.argtypes = [ctypes.c_void_p]
     lib.fake_device_step.restype = ctypes.c_longlong
-    lib.fake_stream.restype = ctypes.c_void_p
+    lib.fake_stream.restype = ctypes.c_void_p  # flags: 1 = cudaStreamNonBlocking
     lib.fake_begin_capture.argtypes = lib.fake_end_capture_and_run.argtypes = [ctypes.c_void_p]
     return lib
 
@@ -139,7 +139,7 @@ def test_a_step_cut_short_leaves_no_forces(fake):
 def _caller_stream(fake, kind):
     if kind == "legacy":
         return 0x1  # cudaStreamLegacy by its handle: cannot be captured
-    return fake.fake_stream()
+    return fake.fake_stream(1)
 
 
 @pytest.mark.parametrize("kind", ["own", "legacy"])
@@ -166,7 +166,7 @@ def test_work_under_a_callers_capture(fake, warm):
     """Evaluations and runs on a stream that the caller is capturing become part of
     the caller's graph, whatever the library would do with them otherwise."""
     s, mask = _system()
-    stream = fake.fake_stream()
+    stream = fake.fake_stream(1)
     s.set_stream(stream)
     if warm:
         for _ in range(6):
@@ -210,4 +210,27 @@ def test_a_launch_shape_can_be_read_and_written_back(fake):
     assert s.launch_shape == dict(default, pme_block=128)
     with pytest.raises(Exception, match="split"):
         s.set_launch_shape(split=3)
+    s.close()
+
+
+@pytest.mark.parametrize("blocking", [True, False])
+def test_a_blocking_stream_is_captured_only_for_runs_that_ask_for_it(fake, blocking):
+    """While a stream that synchronises with the legacy stream is being captured, another
+    thread's work on the legacy stream fails: evaluations and short runs, which come
+    often and ask for no graph, leave such a stream alone."""
+    s, mask = _system()
+    s.set_stream(fake.fake_stream(0 if blocking else 1))
+    for _ in range(8):
+        s.compute_forces(mask)
+        s.integrate(9, mask, want_energy=False)
+    _whole(fake, s, 72)
+    assert (fake.fake_calls(b"cudaStreamBeginCapture") == 0) == blocking
+    s.integrate(250, mask, want_energy=False)
+    _whole(fake, s, 322)
+    assert fake.fake_calls(b"cudaStreamBeginCapture") > 0
+    s.set_graph_mode(1)
+    before = fake.fake_calls(b"cudaGraphLaunch")
+    s.integrate(5, mask, want_energy=False)
+    _whole(fake, s, 327)
+    assert fake.fake_calls(b"cudaGraphLaunch") == before + 5
     s.close()
