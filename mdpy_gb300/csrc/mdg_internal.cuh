@@ -36,8 +36,14 @@ constexpr int kEnergySlots = 16;
 // The pair kernel's default number of work items per cluster, by the size of
 // the cluster's own system, so that a batch member is cut up as it is alone:
 // 4 below this many atoms, 2 from it on.  Alone on the GPU (Ewald, LJ, switch,
-// us at 2 / 4 items): 24k atoms 109 / 88, 48k 153 / 138, 88k 229 / 238, 250k
-// 560 / 625, 500k 1079 / 1188: 2 is clearly ahead only well above 100k atoms.
+// us at 2 / 4 items): 48k atoms 151 / 131, 64k 187 / 162, 80k 205 / 195, 90k 206 /
+// 213, 112k 257 / 257, 135k 294 / 305, 200k 432 / 448, 300k 622 / 667, 600k 1180 /
+// 1316.  The times cross near 85k; the line lies above it (3 % at 90k) because an
+// item's i forces are one FP32 chain, so the count sets their last bits, and runs
+// below the line keep the bits that they have had.  Accuracy is no reason: the
+// chain of 2 items is twice as long, and the force error against FP64 is the same
+// (2 / 4 items: 129k 1.0288e-5 / 1.0282e-5, 200k 9.8561e-6 / 9.8557e-6, 300k
+// 1.3528e-5 / 1.3529e-5, 1M 1.8923e-5 / 1.8924e-5).
 constexpr int kNbLargeSystem = 128000;
 // below this many atoms a system's items may be taken by several warps (the
 // pair kernel's block form), and its sums are cut up accordingly

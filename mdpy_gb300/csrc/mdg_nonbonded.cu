@@ -329,8 +329,10 @@ NbArgs make_args(mdg_system *s) {
 
 }  // namespace
 
-// work items per cluster: as set, or the most that any system's size calls for
-// (LJ without Ewald: always 4)
+// work items per cluster: as set, or the most that any system's size calls for.
+// LJ without Ewald: 4 at every size, which keeps the bits of its FP32 chains (bare
+// Coulomb runs hang on them).  A Lennard-Jones fluid, us at 2 / 4 items: 2,700 atoms
+// 37 / 30.5, 12k 30 / 25, 20k 33 / 32, 80k 81 / 79, but 130k 108 / 117, 300k 231 / 287.
 int nb_parts(const mdg_system *s) {
     if (s->nb_split > 0) return s->nb_split;
     if (s->coul_mode != MDG_COUL_EWALD) return 4;
@@ -365,7 +367,8 @@ cudaError_t launch_nonbonded(mdg_system *s, unsigned mask, int energy, int dump)
     const int coul_tile = (want_c && s->coul_mode == MDG_COUL_EWALD) ? MDG_COUL_EWALD : MDG_COUL_NONE;
     if (want_lj || coul_tile == MDG_COUL_EWALD) {
         // Ewald items of small systems, too few to fill the GPU, are taken by several
-        // warps each (the sums are the same): the most that keep every item with
+        // warps each (the sums are the same; those of LJ without Ewald are FP32
+        // chains, which only one warp can add up in their order): the most that keep every item with
         // work resident (16 warps an SM at this kernel's registers; 4 warps less, as
         // the PME and bonded kernels beside it take room).  A cluster's parts walk
         // batches of 32 clusters, so a system of 64 to 96 has three parts with work.

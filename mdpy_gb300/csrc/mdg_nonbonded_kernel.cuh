@@ -1365,7 +1365,7 @@ __device__ __forceinline__ void nb_item(const NbArgs &a, const int I, const int 
 }
 
 // ---- block form --------------------------------------------------------------
-// A whole-warp item taken by W warps (2, 4 or 8) of one block, for systems
+// A whole-warp item taken by W warps (2, 3, 4 or 8) of one block, for systems
 // whose items alone leave most of the GPU's warp slots empty.  Every warp runs
 // the candidate scan; of each W candidates in scan order warp w loads and tests
 // the w-th, and the survivors are appended to the two rings in candidate order

@@ -20,10 +20,11 @@
 // (small) bin, so a given configuration always yields the same order.  Padding
 // slots carry perm = -1, charge 0 and a far-away position.
 //
-// Bound by launches: 7 dependent kernels of 2 to 5 us (11 kernels and 7 memsets
-// before: one clearing kernel, scans and column tables by one block where they
-// are short, the bin's rank in place of a serial sort per bin, 17 us).  24k
-// atoms 85 -> 33 us, 2,700 82 -> 29, 1M 137 -> 104.
+// Bound by launches: 7 dependent kernels of 2 to 5 us where one block scans the
+// bins (up to 12 x 2048 of them) and builds the column tables (up to 512 columns);
+// two more beyond either limit, 11 for a box of 1M atoms (11 kernels and 7 memsets
+// at every size before: one clearing kernel, the bin's rank in place of a serial
+// sort per bin, 17 us).  24k atoms 85 -> 33 us, 2,700 82 -> 29, 1M 137 -> 104.
 #include <algorithm>
 #include <cmath>
 #include <vector>
